@@ -2,8 +2,9 @@
 
 The product is `lib/libgtok.so` (CUDA kernels + C++ engine + extern "C" boundary,
 built by `python -m graphtok_b200.build`).  This package only locates and binds it
-through ctypes; it has no CPU implementation of the encode path, and `GTok(...)`
-raises when the library or a B200 is missing.
+through ctypes (the calls that take or return Python text, lists and arrays through the extension
+`_host`, which the same build makes); it has no CPU implementation of the encode path, and
+`GTok(...)` raises when the library or a B200 is missing.
 """
 import ctypes
 import os
@@ -96,6 +97,8 @@ def load_lib():
     lib.gtok_x_plan_documents.argtypes = [vp, u32, u32, vp]
     lib.gtok_x_table_bytes.restype = None
     lib.gtok_x_table_bytes.argtypes = [vp, vp]
+    from . import _host                      # built beside the library; it binds to the same libgtok.so
+    lib.host = _host
     lib.gtok_x_launches_per_replay.restype = i32
     lib.gtok_x_launches_per_replay.argtypes = [vp, i32]
     _lib = lib
@@ -112,6 +115,7 @@ class GTok:
     def __init__(self, tokenizer_json, max_bytes=1 << 20):
         self.lib = load_lib()
         self.handle = self.lib.gtok_create(os.fsencode(tokenizer_json), int(max_bytes))
+        self.host = self.lib.host
         if not self.handle:
             raise GTokError("gtok_create failed: %s" % self.lib.gtok_x_last_error().decode("utf-8", "replace"))
         self.max_bytes = max(4096, int(max_bytes))
@@ -137,16 +141,10 @@ class GTok:
 
     def encode(self, data):
         """bytes -> uint32 ids (numpy)."""
-        data = bytes(data)
-        out = np.empty(len(data) + 16, dtype=np.uint32)
-        n = self.lib.gtok_encode(self.handle, data, len(data), out.ctypes.data, out.size)
-        if n == -2:
-            # more ids than bytes: only text that its vocabulary's NFC lengthens (at most threefold)
-            out = np.empty(3 * len(data) + 64, dtype=np.uint32)
-            n = self.lib.gtok_encode(self.handle, data, len(data), out.ctypes.data, out.size)
-        if n < 0:
-            self._fail("gtok_encode", n)
-        return out[:n].copy()
+        ids = self.host.encode(self.handle, data if data.__class__ is bytes else bytes(data), False)
+        if ids.__class__ is int:
+            self._fail("gtok_encode", ids)
+        return ids
 
     def encode_batch(self, blob, offsets):
         """Concatenated documents + n+1 byte offsets -> (ids uint32[T], token offsets uint32[n+1])."""
@@ -162,7 +160,7 @@ class GTok:
             n = self.lib.gtok_encode_batch(self.handle, blob, offsets.ctypes.data, n_docs, out.ctypes.data, out.size, doc.ctypes.data)
         if n < 0:
             self._fail("gtok_encode_batch", n)
-        return out[:n].copy(), doc
+        return out[:n], doc
 
     # ---- measurement -----------------------------------------------------
     def stage(self, blob, offsets=None):
@@ -213,6 +211,12 @@ class GTok:
         """ids -> the bytes they spell, on the device (gtok_x_decode).  `out`: optional uint8 numpy
         buffer to decode into (a page-locked one is written directly); returns bytes, or with
         `want_ms` (bytes, CUDA-event ms of the decode graph)."""
+        if out is None and not want_ms:
+            data = self.host.decode(self.handle, ids)
+            if data.__class__ is bytes:
+                return data
+            if data is not None:
+                self._fail("gtok_x_decode", data)
         ids = np.ascontiguousarray(ids, dtype=np.uint32)
         need = ctypes.c_uint64(0)
         ms = ctypes.c_float(0.0)

@@ -3,6 +3,7 @@
   graphtok_b200/lib/libgtok.so      CUDA kernels + engine + C ABI, sm_100a only
   graphtok_b200/datagen/datagen     synthetic text / vocabulary generator (host only)
   graphtok_b200/cli/gpu_bpe_tokenize   command-line tool over libgtok.so
+  graphtok_b200/_host.so            CPython extension: Python objects to and from libgtok.so
 
 nvcc cross-compiles without a GPU.  Run as `python -m graphtok_b200.build`.
 """
@@ -22,7 +23,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "--shared",
     "-Xlinker", "--version-script=" + os.path.join(CSRC, "gtok.map"),
 ]
-SOURCES = ["encode_kernels.cu", "tiny_kernel.cu", "engine.cu", "gtok_abi.cc", "vocab_host.cc", "tables_build.cc", "nfc_host.cc"]
+SOURCES = ["encode_kernels.cu", "tiny_kernel.cu", "engine.cu", "gtok_abi.cc", "vocab_host.cc", "tables_build.cc", "nfc_host.cc", "host_text.cc", "result_blocks.cc"]
 
 
 def _newer(target, deps):
@@ -80,14 +81,32 @@ def build_cli(force=False):
     return CLI
 
 
+HOST = os.path.join(HERE, "_host.so")
+
+
+def build_host(force=False):
+    """The CPython extension between the Python classes and libgtok.so."""
+    import sysconfig
+
+    import numpy
+    src = os.path.join(HERE, "pyhost", "host_module.cc")
+    if not force and not _newer(HOST, [src, os.path.join(HERE, "..", "include", "gtok.h"), LIB]):
+        return HOST
+    subprocess.run(["g++", "-std=c++17", "-O3", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"], "-I" + numpy.get_include(),
+                    "-o", HOST, src, "-L" + LIB_DIR, "-l:libgtok.so", "-Wl,-rpath,$ORIGIN/lib"], check=True)
+    return HOST
+
+
 def main():
     force = "--force" in sys.argv
     build_lib(force=force, verbose="-v" in sys.argv)
     build_datagen(force=force)
     build_cli(force=force)
+    build_host(force=force)
     print(LIB)
     print(DATAGEN)
     print(CLI)
+    print(HOST)
 
 
 if __name__ == "__main__":

@@ -16,7 +16,9 @@
 
 #include "encode_core.h"
 #include "encode_kernels.h"
+#include "host_text.h"
 #include "nfc_host.h"
+#include "result_blocks.h"
 #include "tables_build.h"
 #include "unicode_class_table.h"
 #include "unicode_wide_table.h"
@@ -134,7 +136,12 @@ private:
 };
 
 constexpr size_t kCopyPart = 512 << 10;      // bytes per staging step: small enough to overlap with the DMA of the one before
+constexpr size_t kSendLeast = 256 << 10;     // bytes of a transfer to the device that does not end the text
 constexpr int kCopyEvents = 64;
+// Characters of a Python string that one step writes out as UTF-8, and the bytes from which such work is
+// shared: at about 4 GB/s a thread it is several times dearer than a copy, so it pays earlier.
+constexpr uint64_t kCharPart = 32 << 10;
+constexpr uint64_t kCharShare = 96 << 10;
 
 constexpr size_t kTextPad = kTile + kWin + 256;
 constexpr uint32_t kHdrWords = 4;     // meta occupies the first 4 words of the header; offsets follow
@@ -251,6 +258,8 @@ struct Engine::Impl {
     const uint8_t* d_tok_blob = nullptr;
     const uint32_t* d_tok16 = nullptr;
     uint32_t max_tok_len = 0;
+    uint32_t decoded = 0;                 // bytes of the last decode that have not been fetched yet
+    std::vector<uint32_t> decode_ids;
     int dec_per_sm = 1;
     Ctx* staged = nullptr;
     int pretok_per_sm = 1, words_per_sm = 1, miss_per_sm = 1, asm_per_sm = 1, nfc_per_sm = 1;
@@ -263,8 +272,28 @@ struct Engine::Impl {
     std::unique_ptr<CopyPool> pool;      // staging copies of large inputs and outputs
     std::unique_ptr<std::atomic<uint8_t>[]> part_done;
     int part_done_n = 0;
+    std::vector<size_t> part_ends;
+    // the pieces of text of one call, cut to what one copy step takes: where each comes from and where it goes
+    struct Slice {
+        const uint8_t* src;
+        uint32_t units, kind;
+        uint64_t off, bytes;
+    };
+    std::vector<Slice> slices;
+    std::vector<uint32_t> part_slices;   // slices up to the end of each step
+    std::vector<uint32_t> text_off;      // batch: where each document begins
+    // a call between put() and take()
+    struct Call {
+        Ctx* c = nullptr;
+        bool tiny = false, batch = false;
+        uint32_t docs = 0, len = 0, cap = 0;
+        int64_t total = -1;
+    } call;
+    uint64_t call_wide = 0;
 
+    Impl() { result_blocks_user(1); }
     ~Impl() {
+        result_blocks_user(-1);
         single.reset();
         batch.reset();
         dec.reset();
@@ -519,6 +548,14 @@ struct Engine::Impl {
     // small, or kNoCtx when the call should take the four-kernel path (the kernel gave up on something).
     int64_t run_tiny(Ctx* c, const uint8_t* text, uint32_t len, uint32_t* out, uint32_t max_out, std::string& err) {
         std::memcpy(c->h_tiny_text, text, len);
+        const int64_t total = launch_tiny_graph(c, len, err);
+        if (total < 0) return total;
+        if (total > max_out) { err = "more token ids than the output buffer holds"; return -2; }
+        std::memcpy(out, c->h_tiny_out, static_cast<size_t>(total) * 4);
+        return total;
+    }
+    // The same for text that is in h_tiny_text already; the ids stay in h_tiny_out.
+    int64_t launch_tiny_graph(Ctx* c, uint32_t len, std::string& err) {
         std::memset(c->h_tiny_text + len, 0, 16);
         c->h_tiny_meta[0] = len;
         c->h_tiny_meta[1] = 1;
@@ -531,10 +568,7 @@ struct Engine::Impl {
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) { err = std::string("short-input graph: ") + cudaGetErrorString(e); return -1; }
         if (reinterpret_cast<volatile uint32_t*>(c->h_status)[1]) return kNoCtx;
-        const uint32_t total = reinterpret_cast<volatile uint32_t*>(c->h_status)[0];
-        if (total > max_out) { err = "more token ids than the output buffer holds"; return -2; }
-        std::memcpy(out, c->h_tiny_out, static_cast<size_t>(total) * 4);
-        return total;
+        return reinterpret_cast<volatile uint32_t*>(c->h_status)[0];
     }
 
     // The two big look-up tables are kept resident in L2 (the reference's tables are "L2-resident" by
@@ -642,8 +676,41 @@ struct Engine::Impl {
         return true;
     }
 
-    // Host -> pinned -> device.  Large inputs piece by piece through the pool: finished pieces go to
-    // the device while the rest is still being copied into pinned memory.
+    // A job of `parts` pieces for the pool and this thread together; piece p fills the bytes [ends[p-1], ends[p])
+    // of the pinned buffer.  Finished pieces go to the device while the rest is still being filled.
+    bool fill_and_send(uint8_t* d_dst, const uint8_t* h_pin, const std::function<void(int)>& fill, const size_t* ends, int parts, cudaStream_t stream,
+                       std::string& err) {
+        if (part_done_n < parts) { part_done.reset(new std::atomic<uint8_t>[parts]); part_done_n = parts; }
+        for (int p = 0; p < parts; ++p) part_done[p].store(0, std::memory_order_relaxed);
+        const std::function<void(int)> fn = [&](int p) {
+            fill(p);
+            part_done[p].store(1, std::memory_order_release);
+        };
+        pool->start(parts, &fn);
+        int issued = 0;
+        size_t sent = 0;
+        cudaError_t ce = cudaSuccess;
+        while (issued < parts) {
+            int upto = issued;
+            while (upto < parts && part_done[upto].load(std::memory_order_acquire)) ++upto;
+            // a transfer starts on a 16-byte line and, but for the last, ends on one: what a part has beyond goes with the next
+            if (upto > issued && (upto == parts || ends[upto - 1] - sent >= kSendLeast)) {
+                const size_t end = upto == parts ? (ends[upto - 1] + 15) & ~size_t(15) : ends[upto - 1] & ~size_t(15);
+                const cudaError_t e1 = cudaMemcpyAsync(d_dst + sent, h_pin + sent, end - sent, cudaMemcpyHostToDevice, stream);
+                if (ce == cudaSuccess) ce = e1;
+                issued = upto;
+                sent = end;
+                continue;
+            }
+            const int p = pool->take();
+            if (p >= 0) { fn(p); pool->done_one(); } else CopyPool::cpu_relax();
+        }
+        pool->finish();
+        if (ce != cudaSuccess) { err = std::string("copy to the device: ") + cudaGetErrorString(ce); return false; }
+        return true;
+    }
+
+    // Host -> pinned -> device, large inputs in pieces.
     bool host_to_device(uint8_t* d_dst, uint8_t* h_pin, const uint8_t* src, size_t len, cudaStream_t stream, std::string& err) {
         if (len >= kCopyPart && is_pinned(src)) {
             // the caller's buffer is page-locked: the device reads it directly, no staging copy (the tail
@@ -658,37 +725,90 @@ struct Engine::Impl {
         }
         if (pool && len >= 2 * kCopyPart) {
             const int parts = static_cast<int>((len + kCopyPart - 1) / kCopyPart);
-            if (part_done_n < parts) { part_done.reset(new std::atomic<uint8_t>[parts]); part_done_n = parts; }
-            for (int p = 0; p < parts; ++p) part_done[p].store(0, std::memory_order_relaxed);
-            const std::function<void(int)> fn = [&](int p) {
+            part_ends.resize(parts);
+            for (int p = 0; p < parts; ++p) part_ends[p] = std::min(static_cast<size_t>(p + 1) * kCopyPart, len);
+            const std::function<void(int)> fill = [&](int p) {
                 const size_t off = static_cast<size_t>(p) * kCopyPart;
                 std::memcpy(h_pin + off, src + off, std::min(kCopyPart, len - off));
-                part_done[p].store(1, std::memory_order_release);
             };
-            pool->start(parts, &fn);
-            int issued = 0;
-            cudaError_t ce = cudaSuccess;
-            while (issued < parts) {
-                int upto = issued;
-                while (upto < parts && part_done[upto].load(std::memory_order_acquire)) ++upto;
-                if (upto > issued) {
-                    const size_t off = static_cast<size_t>(issued) * kCopyPart;
-                    const size_t end = std::min(static_cast<size_t>(upto) * kCopyPart, len);
-                    const cudaError_t e1 = cudaMemcpyAsync(d_dst + off, h_pin + off, (end - off + 15) & ~size_t(15), cudaMemcpyHostToDevice, stream);
-                    if (ce == cudaSuccess) ce = e1;
-                    issued = upto;
-                    continue;
-                }
-                const int p = pool->take();
-                if (p >= 0) { fn(p); pool->done_one(); } else CopyPool::cpu_relax();
-            }
-            pool->finish();
-            if (ce != cudaSuccess) { err = std::string("copy to the device: ") + cudaGetErrorString(ce); return false; }
-        } else {
-            std::memcpy(h_pin, src, len);
-            GTOK_CUDA(cudaMemcpyAsync(d_dst, h_pin, (len + 15) & ~size_t(15), cudaMemcpyHostToDevice, stream));
+            return fill_and_send(d_dst, h_pin, fill, part_ends.data(), parts, stream, err);
         }
+        std::memcpy(h_pin, src, len);
+        GTOK_CUDA(cudaMemcpyAsync(d_dst, h_pin, (len + 15) & ~size_t(15), cudaMemcpyHostToDevice, stream));
         return true;
+    }
+
+    // The pieces of a call as slices with their places in the text; false where a character has no UTF-8 form.
+    // `wide`: characters among them that are not bytes already.
+    bool measure(const TextPiece* pieces, uint32_t n, bool batch, uint64_t* total, uint64_t* wide) {
+        slices.clear();
+        *wide = 0;
+        auto step_of = [](uint32_t kind) { return kind == 1 ? static_cast<uint64_t>(kCopyPart) : kCharPart; };
+        for (uint32_t i = 0; i < n; ++i) {
+            const TextPiece& p = pieces[i];
+            const uint64_t width = p.kind == 2 || p.kind == 4 ? p.kind : 1, step = step_of(p.kind);
+            for (uint64_t at = 0; at < p.units; at += step) {
+                const uint64_t u = std::min(step, p.units - at);
+                slices.push_back({static_cast<const uint8_t*>(p.data) + at * width, static_cast<uint32_t>(u), p.kind, 0, u});
+            }
+            if (p.kind != 1) *wide += p.units;
+        }
+        std::atomic<bool> bad{false};
+        auto size_range = [&](size_t from, size_t to) {
+            for (size_t i = from; i < to; ++i) {
+                Slice& sl = slices[i];
+                if (sl.kind == 1) continue;
+                sl.bytes = utf8_size(sl.src, sl.units, sl.kind);
+                if (sl.bytes == ~0ull) bad.store(true, std::memory_order_relaxed);
+            }
+        };
+        if (pool && *wide >= 4 * kCharPart) {
+            const size_t groups = std::min<size_t>(slices.size(), static_cast<size_t>(*wide / kCharPart));
+            const std::function<void(int)> fn = [&](int g) { size_range(slices.size() * g / groups, slices.size() * (g + 1) / groups); };
+            pool->start(static_cast<int>(groups), &fn);
+            for (int g; (g = pool->take()) >= 0;) { fn(g); pool->done_one(); }
+            pool->finish();
+        } else if (*wide) {
+            size_range(0, slices.size());
+        }
+        if (bad.load()) return false;
+        if (batch) text_off.resize(static_cast<size_t>(n) + 1);
+        uint64_t at = 0;
+        size_t k = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            if (batch) text_off[i] = static_cast<uint32_t>(std::min<uint64_t>(at, 0xFFFFFFFFull));
+            const uint64_t step = step_of(pieces[i].kind);
+            for (uint64_t left = (pieces[i].units + step - 1) / step; left; --left, ++k) { slices[k].off = at; at += slices[k].bytes; }
+        }
+        if (batch) text_off[n] = static_cast<uint32_t>(std::min<uint64_t>(at, 0xFFFFFFFFull));
+        *total = at;
+        return true;
+    }
+    void write_slices(uint8_t* dst, size_t from, size_t to) {
+        for (size_t i = from; i < to; ++i) utf8_write(dst + slices[i].off, slices[i].src, slices[i].units, slices[i].kind);
+    }
+    // The measured slices -> pinned -> device, then the header.
+    bool stage_slices(Ctx* c, uint64_t len, uint64_t wide, const uint32_t* doc_off, uint32_t n_docs, std::string& err) {
+        uint8_t* d_dst = nfc ? c->d_raw : c->d_text;
+        const uint64_t part = wide ? 2 * kCharPart : kCopyPart;
+        if (pool && (wide ? len >= kCharShare : len >= 2 * kCopyPart)) {
+            part_ends.clear();
+            part_slices.clear();
+            uint64_t from = 0;
+            for (size_t i = 0; i < slices.size(); ++i) {
+                const uint64_t end = slices[i].off + slices[i].bytes;
+                if (end - from < part && i + 1 < slices.size()) continue;
+                part_ends.push_back(end);
+                part_slices.push_back(static_cast<uint32_t>(i + 1));
+                from = end;
+            }
+            const std::function<void(int)> fill = [&](int p) { write_slices(c->h_text, p ? part_slices[p - 1] : 0, part_slices[p]); };
+            if (!fill_and_send(d_dst, c->h_text, fill, part_ends.data(), static_cast<int>(part_ends.size()), c->stream, err)) return false;
+        } else if (len) {
+            write_slices(c->h_text, 0, slices.size());
+            GTOK_CUDA(cudaMemcpyAsync(d_dst, c->h_text, (len + 15) & ~size_t(15), cudaMemcpyHostToDevice, c->stream));
+        }
+        return stage_header(c, static_cast<uint32_t>(len), doc_off, n_docs, err, false);
     }
 
     // Host -> pinned -> device, for the text and the header.
@@ -697,6 +817,9 @@ struct Engine::Impl {
                      bool normalised = false) {
         uint8_t* d_dst = nfc ? c->d_raw : c->d_text;
         if (len && !host_to_device(d_dst, c->h_text, bytes, len, c->stream, err)) return false;
+        return stage_header(c, len, doc_off, n_docs, err, normalised);
+    }
+    bool stage_header(Ctx* c, uint32_t len, const uint32_t* doc_off, uint32_t n_docs, std::string& err, bool normalised) {
         c->h_hdr[0] = len;
         c->h_hdr[1] = n_docs;
         c->h_hdr[2] = normalised ? 1u : 0u;
@@ -796,6 +919,12 @@ struct Engine::Impl {
         c = ctx_for(batch_mode, len, n_docs, cap_hint, err);
         if (!c) return kNoCtx;
         if (!stage_input(c, bytes, len, doc_off, n_docs, err)) return -1;
+        return run_staged(c, batch_mode, bytes, len, doc_off, n_docs, cap_hint, err);
+    }
+    // The staged input through the graph.  bytes, len, doc_off: the same input in host memory, which may be the
+    // context's own staging buffers.
+    int64_t run_staged(Ctx*& c, bool batch_mode, const uint8_t* bytes, uint32_t len, const uint32_t* doc_off, uint32_t n_docs,
+                       uint32_t cap_hint, std::string& err) {
         int64_t total = replay(c, false, nullptr, err);
         if (total >= 0 || !nfc || !(last_err_bits & (kErrNfcLong | kErrNfcFull))) return total;
         if (last_err_bits & kErrNfcLong) {
@@ -823,6 +952,10 @@ struct Engine::Impl {
         }
         const uint64_t want = static_cast<uint64_t>(len) * 3 + 64;
         if (want > 0xFFFFFF00ull) { err = "normalised text may exceed 4 GiB"; return -3; }
+        if (bytes == c->h_text) {            // the context, and its staging buffer with it, may be about to go
+            norm.assign(reinterpret_cast<const char*>(bytes), len);
+            bytes = reinterpret_cast<const uint8_t*>(norm.data());
+        }
         c = ctx_for(batch_mode, static_cast<uint32_t>(want), n_docs, cap_hint, err);
         if (!c) return kNoCtx;
         if (!stage_input(c, bytes, len, doc_off, n_docs, err)) return -1;
@@ -977,6 +1110,69 @@ int64_t Engine::encode_batch(const uint8_t* bytes, const uint32_t* doc_off, uint
     return total;
 }
 
+int64_t Engine::measure(const TextPiece* pieces, uint32_t n_pieces, bool batch) {
+    Impl& im = *impl_;
+    im.call = Impl::Call();
+    im.call.batch = batch;
+    im.call.docs = batch ? n_pieces : 1;
+    uint64_t total = 0;
+    if (!im.measure(pieces, n_pieces, batch, &total, &im.call_wide)) return -1;
+    return static_cast<int64_t>(std::min<uint64_t>(total, INT64_MAX));
+}
+
+int64_t Engine::run_measured(uint64_t len64, uint32_t cap_bytes, uint32_t* dev_tokens, uint32_t dev_cap, uint32_t* dev_doc_tok) {
+    Impl& im = *impl_;
+    Impl::Call& cl = im.call;
+    cudaSetDevice(im.device);
+    const uint32_t len = static_cast<uint32_t>(len64);
+    cl.total = -1;
+    cl.c = nullptr;
+    cl.tiny = false;
+    if (len == 0) {
+        if (cl.batch && dev_doc_tok && cudaMemset(dev_doc_tok, 0, (static_cast<size_t>(cl.docs) + 1) * 4) != cudaSuccess) return -1;
+        return cl.total = 0;
+    }
+    const uint32_t* doc_off = cl.batch ? im.text_off.data() : nullptr;
+    cl.c = im.ctx_for(cl.batch, len, cl.docs, cap_bytes, last_error_);
+    if (!cl.c) return cl.batch ? -4 : -1;
+    if (!cl.batch && !dev_tokens && len <= kTinyMaxBytes && cl.c->tiny_exec) {
+        im.write_slices(cl.c->h_tiny_text, 0, im.slices.size());
+        const int64_t r = im.launch_tiny_graph(cl.c, len, last_error_);
+        if (r != Impl::kNoCtx) {
+            cl.tiny = true;
+            return cl.total = r;
+        }
+    }
+    if (!im.stage_slices(cl.c, len, im.call_wide, doc_off, cl.docs, last_error_)) return -1;
+    int64_t total = im.run_staged(cl.c, cl.batch, cl.c->h_text, len, doc_off, cl.docs, cap_bytes, last_error_);
+    if (total == Impl::kNoCtx) return cl.batch ? -4 : -1;
+    if (total < 0) return total;
+    if (im.nfc && cl.c->h_status[2] > cap_bytes) { last_error_ = "normalised text is longer than the handle's byte capacity"; return -3; }
+    if (dev_tokens) {
+        if (static_cast<uint64_t>(total) > dev_cap) { last_error_ = "more token ids than the output buffer holds"; return -2; }
+        cudaError_t e = cudaSuccess;
+        if (total) e = cudaMemcpyAsync(dev_tokens, cl.c->d_out, static_cast<size_t>(total) * 4, cudaMemcpyDeviceToDevice, cl.c->stream);
+        if (e == cudaSuccess && dev_doc_tok)
+            e = cudaMemcpyAsync(dev_doc_tok, cl.c->d_doc_tok, (static_cast<size_t>(cl.docs) + 1) * 4, cudaMemcpyDeviceToDevice, cl.c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cl.c->stream);
+        if (e != cudaSuccess) { last_error_ = std::string("token copy: ") + cudaGetErrorString(e); return -1; }
+    }
+    return cl.total = total;
+}
+
+int Engine::take_ids(uint32_t* out, uint32_t* out_doc_tok) {
+    Impl& im = *impl_;
+    Impl::Call& cl = im.call;
+    if (cl.total < 0) { last_error_ = "no finished call to take the ids of"; return -1; }
+    const size_t total = static_cast<size_t>(cl.total), doc_words = cl.batch ? static_cast<size_t>(cl.docs) + 1 : 0;
+    cl.total = -1;
+    if (!cl.c) { std::memset(out_doc_tok, 0, doc_words * 4); return 0; }
+    if (cl.tiny) { std::memcpy(out, cl.c->h_tiny_out, total * 4); return 0; }
+    if (!total && !doc_words) return 0;
+    cudaSetDevice(im.device);
+    return im.copy_out(cl.c, out, total, out_doc_tok, doc_words, last_error_) ? 0 : -1;
+}
+
 int Engine::stage(const uint8_t* bytes, uint32_t len, const uint32_t* doc_off, uint32_t n_docs, uint32_t cap_bytes) {
     Impl& im = *impl_;
     cudaSetDevice(im.device);
@@ -1110,10 +1306,41 @@ int Engine::read_timeline(unsigned long long* out, uint32_t max_words) {
 
 // ids -> bytes on the device (the reference's TokenizerCtx::decode, src/tokenizer.cu:5499-5573).
 int64_t Engine::decode(const uint32_t* ids, uint32_t n, uint8_t* out, uint64_t max_out, uint64_t* need, float* kernel_ms) {
+    const int64_t total = decode_run(ids, n, max_out, need, kernel_ms);
+    if (total > 0 && take_bytes(out) != 0) return -1;
+    return total;
+}
+
+// A decoding context for `n` ids and `want` bytes, kept or built anew.
+bool Engine::decode_ctx(uint32_t n, uint64_t want) {
+    Impl& im = *impl_;
+    if (im.dec && im.dec->cap_ids >= n && im.dec->cap_bytes >= want) return true;
+    uint32_t cap_ids = 4096;
+    while (cap_ids < n && cap_ids < 0x80000000u) cap_ids <<= 1;
+    if (cap_ids < n) cap_ids = n;
+    size_t cap_bytes = 16384;
+    while (cap_bytes < want) cap_bytes <<= 1;
+    if (im.dec) { cap_ids = std::max(cap_ids, im.dec->cap_ids); cap_bytes = std::max(cap_bytes, im.dec->cap_bytes); }
+    im.dec.reset();
+    if (!im.build_dec(cap_ids, cap_bytes, hv_.vocab_size, last_error_)) { im.dec.reset(); return false; }
+    return true;
+}
+
+uint32_t* Engine::decode_room(uint32_t n) {
+    Impl& im = *impl_;
+    cudaSetDevice(im.device);
+    if (!im.upload_decode_tables(hv_, last_error_)) return nullptr;
+    // (as decode_run wants it, so that the buffer given out here is the one it finds)
+    const uint64_t want = std::min<uint64_t>(std::max<uint64_t>(static_cast<uint64_t>(n) * std::max<uint32_t>(im.max_tok_len, 1), 1024), 16ull * n + 4096);
+    return decode_ctx(n, want) ? im.dec->h_in + 4 : nullptr;
+}
+
+int64_t Engine::decode_run(const uint32_t* ids, uint32_t n, uint64_t max_out, uint64_t* need, float* kernel_ms) {
     Impl& im = *impl_;
     cudaSetDevice(im.device);
     if (need) *need = 0;
     if (kernel_ms) *kernel_ms = 0.f;
+    im.decoded = 0;
     if (n == 0) return 0;
     if (!im.upload_decode_tables(hv_, last_error_)) return -1;
     const uint64_t most = static_cast<uint64_t>(n) * std::max<uint32_t>(im.max_tok_len, 1);
@@ -1126,26 +1353,29 @@ int64_t Engine::decode(const uint32_t* ids, uint32_t n, uint8_t* out, uint64_t m
     DecCtx* c = nullptr;
     uint32_t total = 0, bits = 0;
     for (int attempt = 0; attempt < 2; ++attempt) {
-        if (!im.dec || im.dec->cap_ids < n || im.dec->cap_bytes < want) {
-            uint32_t cap_ids = 4096;
-            while (cap_ids < n && cap_ids < 0x80000000u) cap_ids <<= 1;
-            if (cap_ids < n) cap_ids = n;
-            size_t cap_bytes = 16384;
-            while (cap_bytes < want) cap_bytes <<= 1;
-            if (im.dec) { cap_ids = std::max(cap_ids, im.dec->cap_ids); cap_bytes = std::max(cap_bytes, im.dec->cap_bytes); }
-            im.dec.reset();
-            if (!im.build_dec(cap_ids, cap_bytes, hv_.vocab_size, last_error_)) { im.dec.reset(); return -1; }
+        if (im.dec && ids == im.dec->h_in + 4 && im.dec->cap_bytes < want) {       // the ids are in the buffer that goes with the old context
+            im.decode_ids.assign(ids, ids + n);
+            ids = im.decode_ids.data();
         }
+        if (!decode_ctx(n, want)) return -1;
         c = im.dec.get();
         c->h_in[0] = n;
         c->h_in[1] = c->h_in[2] = c->h_in[3] = 0;
-        cudaError_t e = cudaMemcpyAsync(c->d_in, c->h_in, 16, cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess && !im.host_to_device(reinterpret_cast<uint8_t*>(c->d_in + 4), reinterpret_cast<uint8_t*>(c->h_in + 4),
-                                                   reinterpret_cast<const uint8_t*>(ids), static_cast<size_t>(n) * 4, c->stream, last_error_))
-            return -1;
-        if (e == cudaSuccess) e = cudaEventRecord(c->ev[0], c->stream);
+        const size_t bytes = static_cast<size_t>(n) * 4;
+        cudaError_t e = cudaSuccess;
+        if (ids == c->h_in + 4 || bytes < kCopyPart) {
+            // the count and the ids lie side by side here and on the device: one transfer
+            if (ids != c->h_in + 4) std::memcpy(c->h_in + 4, ids, bytes);
+            e = cudaMemcpyAsync(c->d_in, c->h_in, bytes + 16, cudaMemcpyHostToDevice, c->stream);
+        } else {
+            e = cudaMemcpyAsync(c->d_in, c->h_in, 16, cudaMemcpyHostToDevice, c->stream);
+            if (e == cudaSuccess && !im.host_to_device(reinterpret_cast<uint8_t*>(c->d_in + 4), reinterpret_cast<uint8_t*>(c->h_in + 4),
+                                                       reinterpret_cast<const uint8_t*>(ids), bytes, c->stream, last_error_))
+                return -1;
+        }
+        if (e == cudaSuccess && kernel_ms) e = cudaEventRecord(c->ev[0], c->stream);
         if (e == cudaSuccess) e = cudaGraphLaunch(c->exec, c->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(c->ev[1], c->stream);
+        if (e == cudaSuccess && kernel_ms) e = cudaEventRecord(c->ev[1], c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) { last_error_ = std::string("decode: ") + cudaGetErrorString(e); return -1; }
         if (kernel_ms) cudaEventElapsedTime(kernel_ms, c->ev[0], c->ev[1]);
@@ -1155,20 +1385,31 @@ int64_t Engine::decode(const uint32_t* ids, uint32_t n, uint8_t* out, uint64_t m
         if ((bits & kErrOutputFull) && !(bits & (kErrBadId | kErrWaitExpired)) && total > c->cap_bytes && total <= bound) { want = total; continue; }
         break;
     }
-    cudaError_t e = cudaSuccess;
     if (bits & kErrBadId) { last_error_ = "decode: an id is outside the vocabulary"; return -1; }
     if (bits & kErrWaitExpired) { last_error_ = "decode: a wait on an earlier tile gave up"; return -1; }
     if (total == 0xFFFFFFFFu) { last_error_ = "decode: the ids spell 4 GiB or more, beyond what one call decodes"; return -1; }
     if (need) *need = total;
     if ((bits & kErrOutputFull) || total > max_out) { last_error_ = "decode: more bytes than the output buffer holds"; return -2; }
     if (bits) { last_error_ = "decode: internal error"; return -1; }
-    if (total == 0) return 0;
-    if (im.is_pinned(out)) {
-        e = cudaMemcpyAsync(out, c->d_out, total, cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    } else if (!im.device_to_host(out, c->h_out, c->d_out, total, c->stream, c->out_ev, last_error_)) return -1;
-    if (e != cudaSuccess) { last_error_ = std::string("decode copy: ") + cudaGetErrorString(e); return -1; }
+    im.decoded = total;
     return total;
+}
+
+// The bytes of the last decode_run, to host memory.
+int Engine::take_bytes(uint8_t* out) {
+    Impl& im = *impl_;
+    DecCtx* c = im.dec.get();
+    const uint32_t total = im.decoded;
+    im.decoded = 0;
+    if (!c || !total) { last_error_ = "no finished call to take the bytes of"; return -1; }
+    cudaSetDevice(im.device);
+    if (im.is_pinned(out)) {
+        cudaError_t e = cudaMemcpyAsync(out, c->d_out, total, cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess) { last_error_ = std::string("decode copy: ") + cudaGetErrorString(e); return -1; }
+        return 0;
+    }
+    return im.device_to_host(out, c->h_out, c->d_out, total, c->stream, c->out_ev, last_error_) ? 0 : -1;
 }
 
 const DeviceTables* Engine::device_tables() const { return &impl_->dt; }

@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "host_text.h"
 #include "vocab_host.h"
 
 namespace gtok {
@@ -29,6 +30,22 @@ public:
     // `out_on_device`: out_tokens and out_doc_tok are device pointers, filled by device-to-device copies.
     int64_t encode_batch(const uint8_t* bytes, const uint32_t* doc_off, uint32_t n_docs, uint32_t cap_bytes,
                          uint32_t* out_tokens, uint32_t out_cap, uint32_t* out_doc_tok, bool out_on_device = false);
+
+    // The same call in steps, for callers that hold text in pieces (a list of strings) or make the result's memory
+    // themselves once its size is known:
+    //   measure       the text's UTF-8 bytes; -1 where a character has no UTF-8 form.  With `batch` each piece is a document.
+    //   run_measured  stages the pieces (which must still be in place) and replays; ids stay inside, or go to `dev_tokens`
+    //                 (and `dev_doc_tok`, n_docs + 1 offsets) on the device.  `bytes` is what measure returned.
+    //   take_ids      ids and offsets of the finished call to host memory; 0 or -1.
+    int64_t measure(const TextPiece* pieces, uint32_t n_pieces, bool batch);
+    int64_t run_measured(uint64_t bytes, uint32_t cap_bytes, uint32_t* dev_tokens, uint32_t dev_cap, uint32_t* dev_doc_tok);
+    int take_ids(uint32_t* out, uint32_t* out_doc_tok);
+
+    // Decoding in steps: a page-locked buffer for `n` ids that decode_run then need not copy (optional), the decode
+    // itself, and the bytes it gave to host memory (0 or -1).
+    uint32_t* decode_room(uint32_t n);
+    int64_t decode_run(const uint32_t* ids, uint32_t n, uint64_t max_out, uint64_t* need, float* kernel_ms);
+    int take_bytes(uint8_t* out);
 
     // ids -> the bytes they spell (host buffers).  Returns the byte count, -1 on error (an id outside
     // the vocabulary included), -2 when `max_out` is too small; `need` (optional) receives the byte
@@ -70,6 +87,7 @@ public:
 
 private:
     Engine() = default;
+    bool decode_ctx(uint32_t n, uint64_t want);
     struct Impl;
     std::unique_ptr<Impl> impl_;
     HostVocab hv_;

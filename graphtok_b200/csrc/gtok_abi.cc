@@ -1,6 +1,7 @@
 // extern "C" boundary of libgtok.so; see include/gtok.h for the contract.
 #include "../../include/gtok.h"
 
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -13,6 +14,7 @@
 #include "device_tables.h"
 #include "encode_kernels.h"
 #include "engine.h"
+#include "result_blocks.h"
 #include "shard_plan.h"
 
 namespace {
@@ -340,6 +342,75 @@ int64_t gtok_x_decode(void* handle, const uint32_t* ids, uint32_t n, uint8_t* ou
         if (r < 0) g_last_error = h->engine->last_error();
         return r;
     } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
+}
+
+int64_t gtok_x_measure(void* handle, const gtok_x_piece* pieces, uint32_t n_pieces, int32_t batch) {
+    if (!handle || (!pieces && n_pieces)) return -1;
+    static_assert(sizeof(gtok_x_piece) == sizeof(gtok::TextPiece), "the same layout on both sides of the boundary");
+    try {
+        return static_cast<Handle*>(handle)->engine->measure(reinterpret_cast<const gtok::TextPiece*>(pieces), n_pieces, batch != 0);
+    } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
+}
+
+int64_t gtok_x_encode_measured(void* handle, int64_t bytes, void* out_dev, uint64_t out_cap, void* out_doc_dev) {
+    if (!handle || bytes < 0) return -1;
+    try {
+        Handle* h = static_cast<Handle*>(handle);
+        const uint64_t total = static_cast<uint64_t>(bytes);
+        if (total > 0xFFFFFF00ull) return -3;
+        if (total > h->cap_bytes && (!h->engine->vocab().nfc || total > 3ull * h->cap_bytes)) return -3;      // as in do_encode
+        int64_t n = h->engine->run_measured(total, h->cap_bytes, static_cast<uint32_t*>(out_dev), static_cast<uint32_t>(std::min<uint64_t>(out_cap, 0xFFFFFFFFull)),
+                                            static_cast<uint32_t*>(out_doc_dev));
+        if (n < 0) g_last_error = h->engine->last_error();
+        return n;
+    } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
+}
+
+int32_t gtok_x_take_ids(void* handle, uint32_t* out, uint32_t* out_doc_offsets) {
+    if (!handle) return -1;
+    Handle* h = static_cast<Handle*>(handle);
+    try {
+        const int r = h->engine->take_ids(out, out_doc_offsets);
+        if (r < 0) g_last_error = h->engine->last_error();
+        return r;
+    } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
+}
+
+uint32_t* gtok_x_decode_room(void* handle, uint32_t n) {
+    if (!handle) return nullptr;
+    Handle* h = static_cast<Handle*>(handle);
+    try {
+        uint32_t* p = h->engine->decode_room(n);
+        if (!p) g_last_error = h->engine->last_error();
+        return p;
+    } catch (const std::exception& e) { g_last_error = e.what(); return nullptr; } catch (...) { return nullptr; }
+}
+
+int64_t gtok_x_decode_run(void* handle, const uint32_t* ids, uint32_t n) {
+    if (!handle || (!ids && n)) return -1;
+    Handle* h = static_cast<Handle*>(handle);
+    try {
+        const int64_t r = h->engine->decode_run(ids, n, ~0ull, nullptr, nullptr);
+        if (r < 0) g_last_error = h->engine->last_error();
+        return r;
+    } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
+}
+
+int32_t gtok_x_take_bytes(void* handle, uint8_t* out) {
+    if (!handle || !out) return -1;
+    Handle* h = static_cast<Handle*>(handle);
+    try {
+        const int r = h->engine->take_bytes(out);
+        if (r < 0) g_last_error = h->engine->last_error();
+        return r;
+    } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
+}
+
+void* gtok_x_block_get(uint64_t bytes) {
+    try { return gtok::result_block_get(static_cast<size_t>(bytes)); } catch (...) { return nullptr; }
+}
+void gtok_x_block_put(void* block) {
+    if (block) gtok::result_block_put(block);
 }
 
 int32_t gtok_x_plan_chunks(void* handle, const uint8_t* text, uint64_t len, uint32_t n_parts, uint64_t* out_offsets) {

@@ -32,6 +32,11 @@ def _as_bytes(text):
     raise TypeError("text must be str or bytes")
 
 
+def _device_words(n):
+    import torch
+    return torch.empty(n, dtype=torch.int32, device="cuda")
+
+
 class Tokenizer:
     """One vocabulary, one GPU.  Not thread-safe (same contract as the reference, :1117-1120)."""
 
@@ -39,26 +44,32 @@ class Tokenizer:
         if cpu_backend not in _BACKENDS:
             raise ValueError("cpu_backend must be one of '', 'auto', 'off', 'host', 'gigatoken'")
         self._path = os.fspath(vocab_path)
-        self._cap = max(4096, int(max_input_chars))
-        self._g = GTok(self._path, max_bytes=self._cap)
+        self._g = GTok(self._path, max_bytes=max(4096, int(max_input_chars)))
+        self._host = self._g.host
         self._decode = bool(enable_decode)
         self._staged_docs = None
 
     # ---- capacity ------------------------------------------------------------
+    # The C ABI answers -3 above the handle's byte cap and leaves growing to the caller.  The encode calls below raise
+    # the cap in place as they need it (doubled until three times the text fits, which is the most that NFC makes of
+    # it); the vocabulary and its tables stay as they are.
+    @property
+    def _cap(self):
+        return int(self._g.lib.gtok_x_set_max_bytes(self._g.handle, 0))
+
     def _ensure(self, n_bytes):
-        """The C ABI answers -3 above the handle's byte cap and leaves growing to the caller: the cap
-        is raised in place (gtok_x_set_max_bytes), the vocabulary and its tables stay as they are."""
-        if n_bytes > self._cap:
-            cap = self._cap
+        cap = self._cap
+        if n_bytes > cap:
             while cap < n_bytes:
                 cap *= 2
-            self._cap = self._g.set_max_bytes(cap)
+            self._g.set_max_bytes(cap)
 
     # ---- encode --------------------------------------------------------------
     def encode_numpy(self, text):
-        data = _as_bytes(text)
-        self._ensure(len(data) * 3 + 64)        # NFC lengthens a text at most threefold
-        return self._g.encode(data)
+        ids = self._host.encode(self._g.handle, text, True)
+        if ids.__class__ is int:
+            self._g._fail("gtok_encode", ids)
+        return ids
 
     def encode(self, text):
         return self.encode_numpy(text).tolist()
@@ -66,55 +77,43 @@ class Tokenizer:
     __call__ = encode
 
     def encode_batch(self, texts):
-        texts = list(texts)
+        texts = tuple(texts)
         if not texts:
             return np.zeros(0, dtype=np.uint32), np.zeros(1, dtype=np.uint32)
-        blobs = [_as_bytes(t) for t in texts]
-        offs = np.zeros(len(blobs) + 1, dtype=np.uint32)
-        np.cumsum([len(b) for b in blobs], out=offs[1:])
-        self._ensure(int(offs[-1]) * 3 + 64)
-        return self._g.encode_batch(b"".join(blobs), offs)
+        out = self._host.encode_batch(self._g.handle, texts, True)
+        if out.__class__ is int:
+            self._g._fail("gtok_encode_batch", out)
+        return out
 
     def encode_to_device(self, text):
         """int32 torch tensor on the GPU (torch is imported only here, as in the reference :100-117)."""
-        import torch
-        data = _as_bytes(text)
-        self._ensure(len(data) * 3 + 64)
-        out = torch.empty(len(data) + 16, dtype=torch.int32, device="cuda")
-        n = self._g.lib.gtok_encode_to_device(self._g.handle, data, len(data), ctypes.c_void_p(out.data_ptr()), out.numel())
-        if n == -2:                                 # text its vocabulary's NFC lengthens
-            out = torch.empty(3 * len(data) + 64, dtype=torch.int32, device="cuda")
-            n = self._g.lib.gtok_encode_to_device(self._g.handle, data, len(data), ctypes.c_void_p(out.data_ptr()), out.numel())
-        if n < 0:
-            raise RuntimeError("gtok_encode_to_device returned %d" % n)
-        return out[:n]
+        if text.__class__ is tuple:
+            raise TypeError("text must be str or bytes")
+        out = self._host.encode_to_device(self._g.handle, text, True, _device_words)
+        if out.__class__ is int:
+            raise RuntimeError("gtok_encode_to_device returned %d" % out)
+        return out[0][:out[1]]
 
     def encode_batch_to_device(self, texts):
         """(int32 ids, int32 n+1 token offsets) as torch tensors on the GPU, copied device to device."""
-        import torch
-        blobs = [_as_bytes(t) for t in texts]
-        if not blobs:
+        texts = tuple(texts)
+        if not texts:
+            import torch
             return torch.zeros(0, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
-        offs = np.zeros(len(blobs) + 1, dtype=np.uint32)
-        np.cumsum([len(b) for b in blobs], out=offs[1:])
-        total = int(offs[-1])
-        self._ensure(total * 3 + 64)
-        blob = b"".join(blobs)
-        doc = torch.empty(len(blobs) + 1, dtype=torch.int32, device="cuda")
-        for room in (total + 16, 3 * total + 64):
-            out = torch.empty(room, dtype=torch.int32, device="cuda")
-            n = self._g.lib.gtok_x_encode_batch_to_device(self._g.handle, blob, offs.ctypes.data, len(blobs), ctypes.c_void_p(out.data_ptr()), out.numel(),
-                                                          ctypes.c_void_p(doc.data_ptr()))
-            if n != -2:
-                break
-        if n < 0:
-            raise RuntimeError("gtok_x_encode_batch_to_device returned %d" % n)
-        return out[:n], doc
+        out = self._host.encode_to_device(self._g.handle, texts, True, _device_words)
+        if out.__class__ is int:
+            raise RuntimeError("gtok_encode_batch_to_device returned %d" % out)
+        return out[0][:out[1]], out[2]
 
     # ---- decode (on the device: ids -> the tokens' bytes, gtok_x_decode) ---------
     def decode_bytes(self, ids):
         if not self._decode:
             raise RuntimeError("decode() is disabled; construct Tokenizer(..., enable_decode=True)")
+        data = self._host.decode(self._g.handle, ids)      # lists of int and arrays of 32- and 64-bit integers
+        if data.__class__ is bytes:
+            return data
+        if data is not None:
+            self._g._fail("gtok_x_decode", data)
         arr = np.asarray(ids)
         if arr.size and (arr.min() < 0 or arr.max() > 0xFFFFFFFF):
             raise ValueError("token ids must fit 32 unsigned bits")

@@ -1,0 +1,324 @@
+// graphtok_b200._host: what stands between a Python object and libgtok's calls in steps (gtok_x_measure and
+// what follows it in gtok.h).
+//
+// The library takes text where Python keeps it (a str's own characters, a bytes object's bytes, the strings of a
+// list one by one) and writes ids and bytes to the object that is returned, so a call makes no intermediate
+// Python object and no copy that the transfer to or from the GPU does not need.  Every function takes the
+// handle as an integer and answers an error of the library with its (negative) code as an int.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+#define NPY_NO_DEPRECATED_API NPY_1_7_API_VERSION
+#include <numpy/arrayobject.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <cstring>
+#include <vector>
+
+#include "../../include/gtok.h"
+
+namespace {
+
+// Results from this size on come in page-locked blocks (below it the copy out of the handle's own page-locked
+// buffer takes less than a transfer of its own would).
+constexpr uint64_t kBlockBytes = 256 << 10;
+
+void* handle_of(PyObject* o) { return PyLong_CheckExact(o) ? PyLong_AsVoidPtr(o) : nullptr; }
+
+// The texts of one call: where each lies, and what keeps it there until the call is over.
+struct Texts {
+    std::vector<gtok_x_piece> pieces;
+    std::vector<PyObject*> kept;
+    std::vector<Py_buffer> buffers;
+    gtok_x_piece one;
+    ~Texts() {
+        for (PyObject* o : kept) Py_DECREF(o);
+        for (Py_buffer& b : buffers) PyBuffer_Release(&b);
+    }
+    // False with an exception set: neither str nor bytes-like.
+    bool place(PyObject* o, gtok_x_piece* p) {
+        if (PyUnicode_CheckExact(o)) {
+            p->data = PyUnicode_DATA(o);
+            p->units = static_cast<uint64_t>(PyUnicode_GET_LENGTH(o));
+            const int width = PyUnicode_KIND(o);
+            p->kind = PyUnicode_IS_COMPACT_ASCII(o) ? 1u : width == 1 ? 3u : static_cast<uint32_t>(width);
+            return true;
+        }
+        if (PyBytes_CheckExact(o)) {
+            p->data = PyBytes_AS_STRING(o);
+            p->units = static_cast<uint64_t>(PyBytes_GET_SIZE(o));
+            p->kind = 1;
+            return true;
+        }
+        if (PyByteArray_CheckExact(o) || PyMemoryView_Check(o)) {
+            Py_buffer b;
+            if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) == 0) {
+                buffers.push_back(b);
+                p->data = b.buf;
+                p->units = static_cast<uint64_t>(b.len);
+                p->kind = 1;
+                return true;
+            }
+            PyErr_Clear();          // a view with gaps: its bytes below
+        }
+        PyObject* made = nullptr;
+        if (PyUnicode_Check(o)) made = PyObject_CallMethod(o, "encode", "s", "utf-8");
+        else if (PyBytes_Check(o) || PyByteArray_Check(o) || PyMemoryView_Check(o)) made = PyObject_Bytes(o);
+        else { PyErr_SetString(PyExc_TypeError, "text must be str or bytes"); return false; }
+        if (!made) return false;
+        kept.push_back(made);
+        if (!PyBytes_Check(made)) { PyErr_SetString(PyExc_TypeError, "text must be str or bytes"); return false; }
+        p->data = PyBytes_AS_STRING(made);
+        p->units = static_cast<uint64_t>(PyBytes_GET_SIZE(made));
+        p->kind = 1;
+        return true;
+    }
+};
+
+// The byte cap doubled until a text of `bytes` fits even if normalisation lengthens it (at most threefold).
+void grow_cap(void* h, int64_t bytes) {
+    uint64_t cap = gtok_x_set_max_bytes(h, 0);
+    const uint64_t need = static_cast<uint64_t>(bytes) * 3 + 64;
+    if (!cap || cap >= need) return;
+    while (cap < need) cap *= 2;
+    gtok_x_set_max_bytes(h, static_cast<uint32_t>(std::min<uint64_t>(cap, 0xFFFFFFFFull)));
+}
+
+void release_block(PyObject* capsule) { gtok_x_block_put(PyCapsule_GetPointer(capsule, nullptr)); }
+
+// An array for `n` ids.
+PyObject* new_ids(int64_t n) {
+    npy_intp dim = static_cast<npy_intp>(n);
+    if (static_cast<uint64_t>(n) * 4 >= kBlockBytes) {
+        if (void* p = gtok_x_block_get(static_cast<uint64_t>(n) * 4)) {
+            PyObject* a = PyArray_SimpleNewFromData(1, &dim, NPY_UINT32, p);
+            PyObject* c = a ? PyCapsule_New(p, nullptr, release_block) : nullptr;
+            if (!c) { Py_XDECREF(a); gtok_x_block_put(p); return nullptr; }
+            if (PyArray_SetBaseObject(reinterpret_cast<PyArrayObject*>(a), c) < 0) { Py_DECREF(a); return nullptr; }     // (the capsule is gone either way)
+            return a;
+        }
+    }
+    return PyArray_SimpleNew(1, &dim, NPY_UINT32);
+}
+uint32_t* data_of(PyObject* a) { return static_cast<uint32_t*>(PyArray_DATA(reinterpret_cast<PyArrayObject*>(a))); }
+
+// A character without UTF-8 form is among the texts: the interpreter's own error for it.
+PyObject* raise_encode_error(PyObject* const* objs, Py_ssize_t n) {
+    for (Py_ssize_t i = 0; i < n; ++i) {
+        if (!PyUnicode_Check(objs[i])) continue;
+        PyObject* b = PyUnicode_AsUTF8String(objs[i]);
+        if (!b) return nullptr;
+        Py_DECREF(b);
+    }
+    return PyLong_FromLong(-1);
+}
+
+// Measures and encodes `n` texts; the outcome is the id count, a negative code, or kSurrogate.
+constexpr int64_t kSurrogate = -1000;
+struct Outcome { int64_t bytes, ids; };
+Outcome encode_texts(void* h, const gtok_x_piece* p, uint32_t n, bool batch, bool grow) {
+    Outcome o;
+    Py_BEGIN_ALLOW_THREADS
+    o.bytes = gtok_x_measure(h, p, n, batch ? 1 : 0);
+    if (o.bytes < 0) o.ids = kSurrogate;
+    else {
+        if (grow) grow_cap(h, o.bytes);
+        o.ids = gtok_x_encode_measured(h, o.bytes, nullptr, 0, nullptr);
+    }
+    Py_END_ALLOW_THREADS
+    return o;
+}
+
+// encode(handle, text, grow) -> uint32 array
+PyObject* py_encode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "encode(handle, text, grow)"); return nullptr; }
+    Texts t;
+    if (!t.place(args[1], &t.one)) return nullptr;
+    void* h = handle_of(args[0]);
+    if (!h) return PyLong_FromLong(-1);
+    const Outcome o = encode_texts(h, &t.one, 1, false, args[2] == Py_True);
+    if (o.ids == kSurrogate) return raise_encode_error(args + 1, 1);
+    if (o.ids < 0) return PyLong_FromLongLong(o.ids);
+    PyObject* ids = new_ids(o.ids);
+    if (!ids) return nullptr;
+    int r;
+    if (static_cast<uint64_t>(o.ids) * 4 < kBlockBytes) {
+        r = gtok_x_take_ids(h, data_of(ids), nullptr);
+    } else {
+        Py_BEGIN_ALLOW_THREADS
+        r = gtok_x_take_ids(h, data_of(ids), nullptr);
+        Py_END_ALLOW_THREADS
+    }
+    if (r < 0) { Py_DECREF(ids); return PyLong_FromLong(r); }
+    return ids;
+}
+
+// The texts of a sequence as pieces.  `seq` (from PySequence_Fast on a list or tuple that this call alone holds)
+bool place_all(Texts& t, PyObject* seq) {
+    const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
+    PyObject** items = PySequence_Fast_ITEMS(seq);
+    t.pieces.resize(static_cast<size_t>(n));
+    for (Py_ssize_t i = 0; i < n; ++i)
+        if (!t.place(items[i], &t.pieces[static_cast<size_t>(i)])) return false;
+    return true;
+}
+
+// encode_batch(handle, texts (a tuple, at least one), grow) -> (uint32 ids, uint32 offsets)
+PyObject* py_encode_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 3 || !PyTuple_CheckExact(args[1])) { PyErr_SetString(PyExc_TypeError, "encode_batch(handle, tuple of texts, grow)"); return nullptr; }
+    Texts t;
+    if (!place_all(t, args[1])) return nullptr;
+    void* h = handle_of(args[0]);
+    if (!h) return PyLong_FromLong(-1);
+    const Outcome o = encode_texts(h, t.pieces.data(), static_cast<uint32_t>(t.pieces.size()), true, args[2] == Py_True);
+    if (o.ids == kSurrogate) return raise_encode_error(PySequence_Fast_ITEMS(args[1]), PyTuple_GET_SIZE(args[1]));
+    if (o.ids < 0) return PyLong_FromLongLong(o.ids);
+    PyObject* ids = new_ids(o.ids);
+    if (!ids) return nullptr;
+    npy_intp dim = static_cast<npy_intp>(t.pieces.size()) + 1;
+    PyObject* off = PyArray_SimpleNew(1, &dim, NPY_UINT32);
+    if (!off) { Py_DECREF(ids); return nullptr; }
+    int r;
+    Py_BEGIN_ALLOW_THREADS
+    r = gtok_x_take_ids(h, data_of(ids), data_of(off));
+    Py_END_ALLOW_THREADS
+    if (r < 0) { Py_DECREF(ids); Py_DECREF(off); return PyLong_FromLong(r); }
+    return Py_BuildValue("(NN)", ids, off);
+}
+
+// encode_to_device(handle, text or tuple of texts, grow, make) -> (what make(words) returned for the ids, id count,
+// the same for the offsets or None).  make(words) returns a tensor of that many 32-bit words on the device.
+PyObject* py_encode_to_device(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 4) { PyErr_SetString(PyExc_TypeError, "encode_to_device(handle, text or tuple, grow, make)"); return nullptr; }
+    const bool batch = PyTuple_CheckExact(args[1]);
+    Texts t;
+    if (batch ? !place_all(t, args[1]) : !t.place(args[1], &t.one)) return nullptr;
+    void* h = handle_of(args[0]);
+    if (!h) return PyLong_FromLong(-1);
+    const gtok_x_piece* p = batch ? t.pieces.data() : &t.one;
+    const uint32_t n = batch ? static_cast<uint32_t>(t.pieces.size()) : 1u;
+    int64_t bytes;
+    Py_BEGIN_ALLOW_THREADS
+    bytes = gtok_x_measure(h, p, n, batch ? 1 : 0);
+    if (bytes >= 0 && args[2] == Py_True) grow_cap(h, bytes);
+    Py_END_ALLOW_THREADS
+    if (bytes < 0) return batch ? raise_encode_error(PySequence_Fast_ITEMS(args[1]), PyTuple_GET_SIZE(args[1])) : raise_encode_error(args + 1, 1);
+    auto make = [&](uint64_t words, void** ptr) -> PyObject* {
+        PyObject* w = PyLong_FromUnsignedLongLong(words);
+        PyObject* tensor = w ? PyObject_CallOneArg(args[3], w) : nullptr;
+        Py_XDECREF(w);
+        PyObject* at = tensor ? PyObject_CallMethod(tensor, "data_ptr", nullptr) : nullptr;
+        *ptr = at ? PyLong_AsVoidPtr(at) : nullptr;
+        Py_XDECREF(at);
+        if (PyErr_Occurred()) { Py_XDECREF(tensor); return nullptr; }
+        return tensor;
+    };
+    void *ids_at = nullptr, *off_at = nullptr;
+    PyObject* off = batch ? make(static_cast<uint64_t>(n) + 1, &off_at) : nullptr;
+    if (batch && !off) return nullptr;
+    // one id a byte is the most, but for text that normalisation lengthens (at most threefold)
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        const uint64_t room = attempt ? 3 * static_cast<uint64_t>(bytes) + 64 : static_cast<uint64_t>(bytes) + 16;
+        PyObject* ids = make(room, &ids_at);
+        if (!ids) { Py_XDECREF(off); return nullptr; }
+        int64_t got;
+        Py_BEGIN_ALLOW_THREADS
+        got = gtok_x_encode_measured(h, bytes, ids_at, room, off_at);
+        Py_END_ALLOW_THREADS
+        if (got == -2 && attempt == 0) { Py_DECREF(ids); continue; }
+        if (got < 0) { Py_DECREF(ids); Py_XDECREF(off); return PyLong_FromLongLong(got); }
+        if (!off) { off = Py_None; Py_INCREF(off); }
+        return Py_BuildValue("(NLN)", ids, static_cast<long long>(got), off);
+    }
+    return nullptr;
+}
+
+template <class T>
+bool narrow(const T* s, uint32_t n, uint32_t* d) {
+    uint64_t high = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint64_t v = static_cast<uint64_t>(static_cast<int64_t>(s[i]));
+        high |= v;
+        d[i] = static_cast<uint32_t>(v);
+    }
+    return (high >> 32) == 0;
+}
+
+// decode(handle, ids) -> bytes; None for an `ids` that this function does not take (the caller makes a uint32 array of it)
+PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "decode(handle, ids)"); return nullptr; }
+    void* h = handle_of(args[0]);
+    PyObject* o = args[1];
+    const uint32_t* ids = nullptr;
+    uint32_t n = 0;
+    bool fits = true;
+    if (PyList_CheckExact(o)) {
+        const Py_ssize_t len = PyList_GET_SIZE(o);
+        if (!h || len == 0 || len > 0x3FFFFFFF) Py_RETURN_NONE;
+        n = static_cast<uint32_t>(len);
+        for (Py_ssize_t i = 0; i < len; ++i)
+            if (!PyLong_CheckExact(PyList_GET_ITEM(o, i))) Py_RETURN_NONE;
+        uint32_t* room = gtok_x_decode_room(h, n);
+        if (!room) return PyLong_FromLong(-1);
+        for (Py_ssize_t i = 0; i < len; ++i) {
+            int over = 0;
+            const long long v = PyLong_AsLongLongAndOverflow(PyList_GET_ITEM(o, i), &over);
+            if (over || v < 0 || v > 0xFFFFFFFFll) { fits = false; break; }
+            room[i] = static_cast<uint32_t>(v);
+        }
+        ids = room;
+    } else if (PyArray_CheckExact(o)) {
+        PyArrayObject* a = reinterpret_cast<PyArrayObject*>(o);
+        const npy_intp len = PyArray_SIZE(a);
+        const PyArray_Descr* d = PyArray_DESCR(a);
+        const int width = static_cast<int>(PyArray_ITEMSIZE(a));
+        if (!h || len == 0 || len > 0x3FFFFFFF || !PyArray_IS_C_CONTIGUOUS(a) || !PyArray_ISALIGNED(a) || !PyArray_ISNOTSWAPPED(a) ||
+            (d->kind != 'u' && d->kind != 'i') || (width != 4 && width != 8))
+            Py_RETURN_NONE;
+        n = static_cast<uint32_t>(len);
+        if (d->kind == 'u' && width == 4) ids = static_cast<const uint32_t*>(PyArray_DATA(a));
+        else {
+            uint32_t* room = gtok_x_decode_room(h, n);
+            if (!room) return PyLong_FromLong(-1);
+            const void* s = PyArray_DATA(a);
+            Py_BEGIN_ALLOW_THREADS
+            fits = width == 4 ? narrow(static_cast<const int32_t*>(s), n, room) : narrow(static_cast<const int64_t*>(s), n, room);
+            Py_END_ALLOW_THREADS
+            ids = room;
+        }
+    } else {
+        Py_RETURN_NONE;
+    }
+    if (!fits) { PyErr_SetString(PyExc_ValueError, "token ids must fit 32 unsigned bits"); return nullptr; }
+    int64_t total;
+    Py_BEGIN_ALLOW_THREADS
+    total = gtok_x_decode_run(h, ids, n);
+    Py_END_ALLOW_THREADS
+    if (total < 0) return PyLong_FromLongLong(total);
+    PyObject* bytes = PyBytes_FromStringAndSize(nullptr, static_cast<Py_ssize_t>(total));
+    if (!bytes || total == 0) return bytes;
+    int r;
+    Py_BEGIN_ALLOW_THREADS
+    r = gtok_x_take_bytes(h, reinterpret_cast<uint8_t*>(PyBytes_AS_STRING(bytes)));
+    Py_END_ALLOW_THREADS
+    if (r < 0) { Py_DECREF(bytes); return PyLong_FromLong(r); }
+    return bytes;
+}
+
+PyMethodDef kMethods[] = {
+    {"encode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode)), METH_FASTCALL, "encode(handle, text, grow) -> uint32 array, or an error code"},
+    {"encode_batch", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode_batch)), METH_FASTCALL,
+     "encode_batch(handle, texts, grow) -> (uint32 ids, uint32 offsets), or an error code"},
+    {"encode_to_device", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode_to_device)), METH_FASTCALL,
+     "encode_to_device(handle, text or tuple, grow, make) -> (tensor, id count, offsets or None), or an error code"},
+    {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_decode)), METH_FASTCALL, "decode(handle, ids) -> bytes, None, or an error code"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "Python objects to and from libgtok's calls in steps.", -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) {
+    import_array();
+    return PyModule_Create(&kModule);
+}

@@ -154,6 +154,34 @@ int32_t gtok_x_token_bytes(void* handle, uint32_t id, uint8_t* out, uint32_t cap
  * `kernel_ms` (may be NULL) the CUDA-event time of the graph. */
 int64_t gtok_x_decode(void* handle, const uint32_t* ids, uint32_t n, uint8_t* out, uint64_t max_out, uint64_t* need_out, float* kernel_ms);
 
+/* The encode and decode calls in steps, for bindings that hold text in pieces (a list of strings) and make
+ * the result's memory themselves once its size is known.  A handle takes one call at a time: measure, encode
+ * and take belong together, with nothing else on the handle in between.
+ *   gtok_x_measure         UTF-8 bytes of the pieces, which are the documents of a batch or the parts of one
+ *                          text; -1 where a character has no UTF-8 form (a surrogate)
+ *   gtok_x_encode_measured encodes them (they must still be in place) and returns the id count; return codes as
+ *                          gtok_encode / gtok_encode_batch.  With out_dev the ids (and with out_doc_dev the
+ *                          n_pieces + 1 token offsets of a batch) go to device memory, else gtok_x_take_ids
+ *                          copies them to host memory (directly where that is page-locked)
+ *   gtok_x_decode_room     a page-locked buffer for n ids; ids put there need no further copy.  Optional
+ *   gtok_x_decode_run      ids -> bytes, which gtok_x_take_bytes copies to host memory; returns their number
+ *   gtok_x_block_get       page-locked memory for a result, from a bounded pool shared by all handles and
+ *                          threads; NULL when the pool is exhausted (use ordinary memory then)
+ */
+typedef struct {
+    const void* data;
+    uint64_t units;      /* bytes (kind 1) or characters */
+    uint32_t kind;       /* 1 bytes as they are (UTF-8 or whatever the text is); characters of 2 or 4 bytes: 2, 4; of one byte (Latin-1): 3 */
+} gtok_x_piece;
+int64_t gtok_x_measure(void* handle, const gtok_x_piece* pieces, uint32_t n_pieces, int32_t batch);
+int64_t gtok_x_encode_measured(void* handle, int64_t bytes, void* out_dev, uint64_t out_cap, void* out_doc_dev);
+int32_t gtok_x_take_ids(void* handle, uint32_t* out, uint32_t* out_doc_offsets);
+uint32_t* gtok_x_decode_room(void* handle, uint32_t n);
+int64_t gtok_x_decode_run(void* handle, const uint32_t* ids, uint32_t n);
+int32_t gtok_x_take_bytes(void* handle, uint8_t* out);
+void* gtok_x_block_get(uint64_t bytes);
+void gtok_x_block_put(void* block);
+
 /* Partitioning over the GPUs of one box (no counterpart in the reference, which is
  * single-GPU).  gtok_x_plan_chunks cuts one document into n_parts pieces at
  * positions where a pre-token starts whatever precedes it (letter | space letter),

@@ -1,0 +1,132 @@
+"""The way of Python objects to the library and back: UTF-8 form of a str's characters (CPU), and the calls of
+gpu_bpe_tokenizer that take text and ids as Python holds them (GPU), each against the interpreter's own UTF-8
+form encoded by the same handle from one bytes object, or against the oracle."""
+import ctypes
+import os
+import random
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT, tiny_vocab
+
+WIDTH = {"ascii": (0x20, 0x7E), "latin1": (0xA0, 0xFF), "ucs2": (0x400, 0xD7FF), "ucs4": (0x1F300, 0x1F5FF)}
+
+
+def _text(kind, n, seed):
+    rng = random.Random("%s %d %d" % (kind, n, seed))
+    lo, hi = WIDTH[kind]
+    out = [chr(rng.randint(lo, hi)) if rng.random() < 0.4 else chr(rng.choice((32, 97, 101, 110, 116, 10))) for _ in range(n)]
+    if n:
+        out[rng.randrange(n)] = chr(hi)        # the str has the width its kind stands for
+    return "".join(out)
+
+
+@pytest.fixture(scope="module")
+def utf8(tmp_path_factory):
+    d = tmp_path_factory.mktemp("utf8")
+    src = d / "wrap.cc"
+    src.write_text('#include "host_text.h"\n'
+                   'extern "C" unsigned long long size(const void* p, unsigned long long n, unsigned k) { return gtok::utf8_size(p, n, k); }\n'
+                   'extern "C" unsigned long long put(unsigned char* d, const void* p, unsigned long long n, unsigned k) { return gtok::utf8_write(d, p, n, k) - d; }\n')
+    csrc = os.path.join(ROOT, "graphtok_b200", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-O3", "-fPIC", "-shared", "-I" + csrc, "-o", str(d / "wrap.so"), str(src), os.path.join(csrc, "host_text.cc")], check=True)
+    lib = ctypes.CDLL(str(d / "wrap.so"))
+    lib.size.restype = lib.put.restype = ctypes.c_ulonglong
+    lib.size.argtypes = [ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint]
+    lib.put.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint]
+    return lib
+
+
+@pytest.mark.parametrize("width,kind", [(1, 3), (2, 2), (4, 4)])
+@pytest.mark.parametrize("n", [0, 1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 79, 80, 127, 128, 129, 1000])
+def test_utf8_form(utf8, width, kind, n):
+    """Every length class of characters at the edges of the 16-, 32- and 64-character steps; nothing written past the end."""
+    rng = np.random.default_rng(n * 8 + width)
+    top = {1: 0xFF, 2: 0xFFFF, 4: 0x10FFFF}[width]
+    for mode in range(6):
+        limit = [0x7F, 0x80, 0x7FF, 0x800, 0xFFFF, top][mode]
+        cps = rng.integers(0, min(limit, top) + 1, n)
+        cps[(cps >= 0xD800) & (cps < 0xE000)] = 0xE000 if top > 0xFF else 0x41
+        units = cps.astype({1: np.uint8, 2: np.uint16, 4: np.uint32}[width])
+        want = "".join(map(chr, cps)).encode("utf-8")
+        assert utf8.size(units.ctypes.data, n, kind) == len(want)
+        out = np.full(len(want) + 80, 0xAA, dtype=np.uint8)
+        assert utf8.put(out.ctypes.data, units.ctypes.data, n, kind) == len(want)
+        assert out[:len(want)].tobytes() == want and (out[len(want):] == 0xAA).all()
+        if n and width > 1:
+            units[n // 2] = 0xDC00
+            assert utf8.size(units.ctypes.data, n, kind) == 0xFFFFFFFFFFFFFFFF
+
+
+@pytest.fixture(scope="module")
+def tok():
+    from graphtok_b200.gpu_bpe_tokenizer import Tokenizer
+    return Tokenizer(tiny_vocab("llama3"))
+
+
+# sizes: single-block route and its limit, one copy step and several, the size from which characters are shared among
+# threads, results below and above the size of a page-locked block
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", list(WIDTH))
+@pytest.mark.parametrize("n", [0, 1, 33, 2047, 2049, 40000, 70001, 400003])
+def test_str_and_bytes_alike(tok, oracles, kind, n):
+    text = _text(kind, n, 1)
+    data = text.encode("utf-8")
+    want = oracles["llama3"].encode(data)
+    for form in (text, data, bytearray(data), memoryview(data), memoryview(data[::-1])[::-1]):
+        got = tok.encode_numpy(form)
+        assert got.dtype == np.uint32 and got.flags.writeable and np.array_equal(got, want)
+    assert np.array_equal(tok.encode_to_device(text).cpu().numpy(), want)
+    assert tok.decode_bytes(want) == tok._g.decode(want.astype(np.int64)) == data
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("docs,longest", [(1, 50), (7, 0), (300, 40), (40, 30000), (3, 300000)])
+def test_batch_of_mixed_objects(tok, oracles, docs, longest):
+    rng = random.Random(docs)
+    texts = [_text(rng.choice(list(WIDTH)), rng.randint(0, longest), i) for i in range(docs)]
+    form = (lambda s: s, lambda s: s.encode(), lambda s: bytearray(s.encode()), lambda s: memoryview(s.encode()))
+    ids, off = tok.encode_batch(form[i % 4](s) for i, s in enumerate(texts))
+    want = [oracles["llama3"].encode(s.encode()) for s in texts]
+    assert off.tolist() == np.concatenate([[0], np.cumsum([w.size for w in want])]).tolist()
+    assert np.array_equal(ids, np.concatenate(want))
+    dev, dev_off = tok.encode_batch_to_device(texts)
+    assert np.array_equal(dev.cpu().numpy(), ids.astype(np.int32)) and dev_off.cpu().tolist() == off.tolist()
+
+
+@pytest.mark.gpu
+def test_results_outlive_later_calls(tok, oracles):
+    """More large results at once than there are page-locked blocks: each stays as it was."""
+    texts = [_text("ucs2", 120000, i) for i in range(9)]
+    got = [tok.encode_numpy(t) for t in texts]
+    for t, g in zip(texts, got):
+        assert np.array_equal(g, oracles["llama3"].encode(t.encode()))
+    part = got[0][5:9]
+    keep = part.tolist()
+    del got
+    tok.encode_numpy(texts[8])
+    assert part.tolist() == keep
+
+
+@pytest.mark.gpu
+def test_refused_inputs(tok):
+    for bad in (3, None, [1], ("a",)):
+        with pytest.raises(TypeError):
+            tok.encode_numpy(bad)
+        with pytest.raises(TypeError):
+            tok.encode_batch(["a", bad])
+        with pytest.raises(TypeError):
+            tok.encode_to_device(bad)
+    for lone in ("\ud800", "a" * 100 + "\udfff" + "b" * 100, "\U0001F600\udc00"):
+        with pytest.raises(UnicodeEncodeError):
+            tok.encode_numpy(lone)
+        with pytest.raises(UnicodeEncodeError):
+            tok.encode_batch(["fine", lone])
+    for bad in ([5, -1], [1 << 32], np.array([-1], dtype=np.int32), np.array([1 << 32]), np.array([1 << 32], dtype=np.uint64)):
+        with pytest.raises(ValueError):
+            tok.decode_bytes(bad)
+    for ids in ([72, 105], [True, 3], np.array([[72, 105]], dtype=np.uint16), np.arange(40)[::2], np.arange(9, dtype=np.int32), (7, 8), []):
+        assert tok.decode_bytes(ids) == tok._g.decode(np.asarray(ids).astype(np.uint32).reshape(-1), want_ms=True)[0]
+    assert tok.encode_numpy("still works").size > 0
