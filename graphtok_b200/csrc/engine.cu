@@ -137,6 +137,7 @@ private:
 
 constexpr size_t kCopyPart = 512 << 10;      // bytes per staging step: small enough to overlap with the DMA of the one before
 constexpr size_t kSendLeast = 256 << 10;     // bytes of a transfer to the device that does not end the text
+constexpr size_t kStreamLeast = 64 << 10;    // bytes from which text is staged past the caches
 constexpr int kCopyEvents = 64;
 // Characters of a Python string that one step writes out as UTF-8, and the bytes from which such work is
 // shared: at about 4 GB/s a thread it is several times dearer than a copy, so it pays earlier.
@@ -729,7 +730,7 @@ struct Engine::Impl {
             for (int p = 0; p < parts; ++p) part_ends[p] = std::min(static_cast<size_t>(p + 1) * kCopyPart, len);
             const std::function<void(int)> fill = [&](int p) {
                 const size_t off = static_cast<size_t>(p) * kCopyPart;
-                std::memcpy(h_pin + off, src + off, std::min(kCopyPart, len - off));
+                utf8_stream(h_pin + off, src + off, std::min(kCopyPart, len - off), 1);
             };
             return fill_and_send(d_dst, h_pin, fill, part_ends.data(), parts, stream, err);
         }
@@ -787,6 +788,9 @@ struct Engine::Impl {
     void write_slices(uint8_t* dst, size_t from, size_t to) {
         for (size_t i = from; i < to; ++i) utf8_write(dst + slices[i].off, slices[i].src, slices[i].units, slices[i].kind);
     }
+    void stream_slices(uint8_t* dst, size_t from, size_t to) {
+        for (size_t i = from; i < to; ++i) utf8_stream(dst + slices[i].off, slices[i].src, slices[i].units, slices[i].kind);
+    }
     // The measured slices -> pinned -> device, then the header.
     bool stage_slices(Ctx* c, uint64_t len, uint64_t wide, const uint32_t* doc_off, uint32_t n_docs, std::string& err) {
         uint8_t* d_dst = nfc ? c->d_raw : c->d_text;
@@ -802,10 +806,10 @@ struct Engine::Impl {
                 part_slices.push_back(static_cast<uint32_t>(i + 1));
                 from = end;
             }
-            const std::function<void(int)> fill = [&](int p) { write_slices(c->h_text, p ? part_slices[p - 1] : 0, part_slices[p]); };
+            const std::function<void(int)> fill = [&](int p) { stream_slices(c->h_text, p ? part_slices[p - 1] : 0, part_slices[p]); };
             if (!fill_and_send(d_dst, c->h_text, fill, part_ends.data(), static_cast<int>(part_ends.size()), c->stream, err)) return false;
         } else if (len) {
-            write_slices(c->h_text, 0, slices.size());
+            if (len >= kStreamLeast) stream_slices(c->h_text, 0, slices.size()); else write_slices(c->h_text, 0, slices.size());
             GTOK_CUDA(cudaMemcpyAsync(d_dst, c->h_text, (len + 15) & ~size_t(15), cudaMemcpyHostToDevice, c->stream));
         }
         return stage_header(c, static_cast<uint32_t>(len), doc_off, n_docs, err, false);

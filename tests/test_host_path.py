@@ -29,18 +29,20 @@ def utf8(tmp_path_factory):
     src = d / "wrap.cc"
     src.write_text('#include "host_text.h"\n'
                    'extern "C" unsigned long long size(const void* p, unsigned long long n, unsigned k) { return gtok::utf8_size(p, n, k); }\n'
-                   'extern "C" unsigned long long put(unsigned char* d, const void* p, unsigned long long n, unsigned k) { return gtok::utf8_write(d, p, n, k) - d; }\n')
+                   'extern "C" unsigned long long put(unsigned char* d, const void* p, unsigned long long n, unsigned k) { return gtok::utf8_write(d, p, n, k) - d; }\n'
+                   'extern "C" unsigned long long stream(unsigned char* d, const void* p, unsigned long long n, unsigned k) { return gtok::utf8_stream(d, p, n, k) - d; }\n')
     csrc = os.path.join(ROOT, "graphtok_b200", "csrc")
     subprocess.run(["g++", "-std=c++17", "-O3", "-fPIC", "-shared", "-I" + csrc, "-o", str(d / "wrap.so"), str(src), os.path.join(csrc, "host_text.cc")], check=True)
     lib = ctypes.CDLL(str(d / "wrap.so"))
-    lib.size.restype = lib.put.restype = ctypes.c_ulonglong
+    lib.size.restype = lib.put.restype = lib.stream.restype = ctypes.c_ulonglong
     lib.size.argtypes = [ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint]
     lib.put.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint]
+    lib.stream.argtypes = lib.put.argtypes
     return lib
 
 
 @pytest.mark.parametrize("width,kind", [(1, 3), (2, 2), (4, 4)])
-@pytest.mark.parametrize("n", [0, 1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 79, 80, 127, 128, 129, 1000])
+@pytest.mark.parametrize("n", [0, 1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 79, 80, 127, 128, 129, 1000, 1025, 3000])
 def test_utf8_form(utf8, width, kind, n):
     """Every length class of characters at the edges of the 16-, 32- and 64-character steps; nothing written past the end."""
     rng = np.random.default_rng(n * 8 + width)
@@ -55,6 +57,10 @@ def test_utf8_form(utf8, width, kind, n):
         out = np.full(len(want) + 80, 0xAA, dtype=np.uint8)
         assert utf8.put(out.ctypes.data, units.ctypes.data, n, kind) == len(want)
         assert out[:len(want)].tobytes() == want and (out[len(want):] == 0xAA).all()
+        for at in (0, 1, 63, 64):                # wherever in a line the destination begins
+            out = np.full(at + len(want) + 80, 0xAA, dtype=np.uint8)
+            assert utf8.stream(out.ctypes.data + at, units.ctypes.data, n, kind) == len(want)
+            assert out[at:at + len(want)].tobytes() == want and (out[:at] == 0xAA).all() and (out[at + len(want):] == 0xAA).all()
         if n and width > 1:
             units[n // 2] = 0xDC00
             assert utf8.size(units.ctypes.data, n, kind) == 0xFFFFFFFFFFFFFFFF
