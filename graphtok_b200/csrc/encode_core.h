@@ -8,7 +8,9 @@
 //                   their id in the tile's slot array (one u32 per byte, id at the byte where the
 //                   pre-token starts), unknown ones go to global lists by length class.
 //   miss_batch    : a batch of unknown pre-tokens of one length class: greedy merge loop, one
-//                   thread per pre-token, over a shared-memory symbol arena.
+//                   thread per pre-token, over a shared-memory symbol arena (the throughput form).
+//   miss_teams    : the same for texts with few unknown pre-tokens: 4 to 16 lanes per pre-token, many
+//                   merges in one round (the latency form).
 //   long_word     : one pre-token of more than 64 bytes, by a whole block (run-length merge for
 //                   runs of one character, round-batched merge otherwise).
 //   assemble_tile : the tile's slots -> ids at their final place in the output.
@@ -16,6 +18,7 @@
 // All are written against a small "thread block" interface (Blk):
 //     blk.par(f)                run f(tid) for every thread, then barrier
 //     blk.excl_scan(arr,total)  in-place exclusive scan of arr[kThreads]
+//     blk.warps(f)              run f(warp) for every warp, then barrier; warp.lanes(f) runs f(lane) for its lanes
 //     blk.lookback(st,tile,total,ctl)  publish this tile's total, return the sum of all earlier tiles'
 // so that the CUDA kernels in encode_kernels.cu (one real thread per tid) and a
 // serial emulation used by the CPU tests execute the very same logic.  Nothing
@@ -31,14 +34,18 @@
 #pragma once
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "device_tables.h"
 
 #if defined(__CUDACC__)
 #define GTOK_DEV __device__ __forceinline__
 #define GTOK_DEV_NOINLINE static __device__ __noinline__
+#define GTOK_UNROLL _Pragma("unroll")
 #else
 #define GTOK_DEV inline
 #define GTOK_DEV_NOINLINE inline
+#define GTOK_UNROLL
 #endif
 
 namespace gtok {
@@ -290,32 +297,6 @@ GTOK_DEV unsigned long long wait_state(const unsigned long long* st, int j, uint
     }
     global_or(ctl + 2, kErrWaitExpired);
     return kStFinal;
-}
-
-// Counts one more finished producer, after everything this block wrote before (the caller has
-// passed a block barrier since).
-GTOK_DEV void release_add(uint32_t* p, uint32_t v) {
-#if defined(__CUDA_ARCH__)
-    __threadfence();
-    atomicAdd(p, v);
-#else
-    *p += v;
-#endif
-}
-// Waits until the counter reaches `want`; false (and the error bit) when the limit runs out.
-GTOK_DEV bool wait_count(const uint32_t* p, uint32_t want, uint32_t* ctl) {
-    for (int it = 0; it < kWaitLimit; ++it) {
-#if defined(__CUDA_ARCH__)
-        uint32_t v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-#else
-        const uint32_t v = *p;
-#endif
-        if (v >= want) return true;
-        backoff(); backoff(); backoff(); backoff();       // many blocks poll this one word
-    }
-    global_or(ctl + 2, kErrWaitExpired);
-    return false;
 }
 
 // ---- merge-rule probe ----------------------------------------------------------
@@ -2252,10 +2233,7 @@ constexpr int kMissBatch = kThreads / 2;       // unknown pre-tokens per batch o
 constexpr int kArenaSyms = 3072;               // symbols of one batch (ids, ranks, results: 36 KB)
 constexpr int kSumTiles = 16384;               // documents up to this many tiles (64 MiB): tile bases by direct summation
 constexpr int kLongPerTile = 64;               // a tile holds fewer than 4096 / 65 pre-tokens longer than 64 bytes
-enum { CTL_PRETOK = 0, CTL_ASM = 1, CTL_ERR = 2, CTL_EXIT = 3, CTL_NMISS = 4, CTL_NLONG = 5, CTL_BATCH = 6, CTL_LONG = 7, CTL_NMED = 8, CTL_NFC = 9, CTL_NMED2 = 10, CTL_NMED1 = 11, CTL_NFCFLAG = 12,
-       CTL_FILTERED = 13,   // calls of the 17..32-byte class that are through their whole-token lookups (surplus handed back)
-       CTL_SURPLUS = 14,    // ticket for the chunks of that surplus
-       CTL_NSURPLUS = 15 }; // entries handed back in all
+enum { CTL_PRETOK = 0, CTL_ASM = 1, CTL_ERR = 2, CTL_EXIT = 3, CTL_NMISS = 4, CTL_NLONG = 5, CTL_BATCH = 6, CTL_LONG = 7, CTL_NMED = 8, CTL_NFC = 9, CTL_NMED2 = 10, CTL_NMED1 = 11, CTL_NFCFLAG = 12 };
 constexpr int kShortWordMax = 16;              // unknown pre-tokens up to this length and the longer ones are batched apart
 // A batch lasts as long as its longest merge chain, so pre-tokens are batched by length class and
 // the classes are handed out longest first: 49..64 bytes, 33..48, 17..32, then the short ones.
@@ -2286,7 +2264,7 @@ struct MissSmem {
     alignas(16) uint32_t ws[3 * kArenaSyms];   // arena: ids, ranks, results (also the long pre-token workspace)
     uint32_t b2i[256];
     unsigned long long word[kThreads]; // this batch's entries of the global list (0 = none, or done already)
-    unsigned long long cand[kThreads]; // list entries left over after the whole-token look-up
+    unsigned long long cand[kThreads]; // a call's list entries; then those left over after the whole-token look-up
     alignas(16) uint16_t lnk[kArenaSyms];   // live-symbol chain of each pre-token (prev << 8 | next)
     alignas(16) uint32_t gmin[kArenaSyms / 4];   // lowest rank key of each group of four slots, laid out like the arena (pre-tokens of more than 16 bytes)
     uint8_t rawb[kArenaSyms];          // the pre-tokens' text bytes, max_len apart
@@ -2867,18 +2845,45 @@ GTOK_DEV void arena_pairs(Blk& blk, const EncodeArgs& a, MissSmem& sm, uint32_t*
     }
 }
 
+// The bytes of `n` list entries to shared memory, `max_len` apart: all threads, a word each, so that the loads overlap.
+template <class Blk>
+GTOK_DEV void stage_entries(Blk& blk, const EncodeArgs& a, const unsigned long long* entries, uint32_t n, uint32_t max_len, uint8_t* stage_bytes) {
+    blk.par([&](int tid) {
+        // (a word of four bytes per load where the address allows, and four loads in flight per thread:
+        // a plain byte loop waits for every byte in turn, thirty-two memory round trips in a row)
+        const uint32_t words_per = max_len / 4u;
+        for (uint32_t x0 = tid; x0 < n * words_per; x0 += 4 * kThreads) {
+            uint32_t v[4];
+            GTOK_UNROLL
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t x = x0 + u * kThreads;
+                v[u] = 0;
+                if (x >= n * words_per) continue;
+                const uint32_t w = x / words_per, r = (x % words_per) * 4u;
+                const unsigned long long wv = entries[w];
+                const uint32_t g = static_cast<uint32_t>(wv), len = static_cast<uint32_t>(wv >> 32);
+                if (r >= len || len <= static_cast<uint32_t>(kWordKeyMax)) continue;      // (shorter ones the whole-word table has answered for)
+                const uint8_t* p = a.text + g + r;
+                if (r + 4u <= len && (reinterpret_cast<uintptr_t>(p) & 3u) == 0) v[u] = ldg(reinterpret_cast<const uint32_t*>(p));
+                else for (uint32_t b = 0; b < 4u && r + b < len; ++b) v[u] |= static_cast<uint32_t>(ldg(p + b)) << (8 * b);
+            }
+            GTOK_UNROLL
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t x = x0 + u * kThreads;
+                if (x < n * words_per) reinterpret_cast<uint32_t*>(stage_bytes)[x] = v[u];     // bytes past the entry's end are never read
+            }
+        }
+    });
+}
+
 // ---- kernel 3a: one batch of unknown pre-tokens (2..64 bytes), one per thread ----------
 // All threads fetch the batch's bytes into the block's arena and probe the initial pairs, a
 // slot each; then the thread that owns a pre-token merges it (lowest rank first) and stores
 // the ids.  `max_len` is the longest pre-token of the batch's length class: batch * max_len
 // slots fit the arena.
-// kMode 1 (`share`): a call with take > batch hands back what it cannot merge in one arena; kMode 2
-// (`surplus`): the entries are such handed-back ones.  (Template values, so that the plain call's code is
-// what it was without them.)
-template <class Blk, int kMode = 0>
+template <class Blk>
 GTOK_DEV void miss_batch(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsigned long long* list, int dir, uint32_t first, uint32_t n_miss,
                          uint32_t batch, uint32_t max_len, uint32_t take) {
-    constexpr bool share = kMode == 1, surplus = kMode == 2;
     const DeviceTables& tb = a.tb;
     uint32_t* ids = sm.ws;
     uint32_t* rk = sm.ws + kArenaSyms;
@@ -2918,36 +2923,7 @@ GTOK_DEV void miss_batch(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsi
             if (tid == 0) sm.ctr[C_USED] = 0;
             if (static_cast<uint32_t>(tid) < n_take) sm.cand[tid] = list[static_cast<long long>(dir) * static_cast<long long>(first + tid)];
         });
-        blk.par([&](int tid) {
-            // (a word of four bytes per load where the address allows, and four loads in flight per thread:
-            // a plain byte loop waits for every byte in turn, thirty-two memory round trips in a row)
-            const uint32_t words_per = max_len / 4u;
-            for (uint32_t x0 = tid; x0 < n_take * words_per; x0 += 4 * kThreads) {
-                uint32_t v[4];
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-                for (int u = 0; u < 4; ++u) {
-                    const uint32_t x = x0 + u * kThreads;
-                    v[u] = 0;
-                    if (x >= n_take * words_per) continue;
-                    const uint32_t w = x / words_per, r = (x % words_per) * 4u;
-                    const unsigned long long wv = sm.cand[w];
-                    const uint32_t g = static_cast<uint32_t>(wv), len = static_cast<uint32_t>(wv >> 32);
-                    if (r >= len) continue;
-                    const uint8_t* p = a.text + g + r;
-                    if (r + 4u <= len && (reinterpret_cast<uintptr_t>(p) & 3u) == 0) v[u] = ldg(reinterpret_cast<const uint32_t*>(p));
-                    else for (uint32_t b = 0; b < 4u && r + b < len; ++b) v[u] |= static_cast<uint32_t>(ldg(p + b)) << (8 * b);
-                }
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-                for (int u = 0; u < 4; ++u) {
-                    const uint32_t x = x0 + u * kThreads;
-                    if (x < n_take * words_per) reinterpret_cast<uint32_t*>(stage_bytes)[x] = v[u];     // bytes past the entry's end are never read
-                }
-            }
-        });
+        stage_entries(blk, a, sm.cand, n_take, max_len, stage_bytes);
         typename Blk::template Local<unsigned long long> left;
         blk.par([&](int tid) {
             left.at(tid) = 0ull;
@@ -2963,38 +2939,19 @@ GTOK_DEV void miss_batch(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsi
             if (wv) sm.cand[shared_add(&sm.ctr[C_USED], 1u)] = wv;
         });
         n_cand = sm.ctr[C_USED];
-        if (share) {
-            // What does not fit one arena goes back to the head of this call's stretch of the list, its
-            // count in front of it, for whichever block is free first (miss_surplus): a text whose long
-            // pre-tokens are not in the vocabulary would otherwise keep this block for three arenas in a row.
-            const uint32_t extra = n_cand > batch ? n_cand - batch : 0u;
-            unsigned long long* wlist = const_cast<unsigned long long*>(list);
-            blk.par([&](int tid) {
-                if (tid == 0) store_state(wlist + static_cast<long long>(dir) * static_cast<long long>(first), extra);
-                if (static_cast<uint32_t>(tid) < extra)
-                    store_state(wlist + static_cast<long long>(dir) * static_cast<long long>(first + 1u + tid), sm.cand[batch + tid]);
-            });
-            blk.par([&](int tid) {
-                if (tid != 0) return;
-                if (extra) global_add(a.ctl + CTL_NSURPLUS, extra);
-                release_add(a.ctl + CTL_FILTERED, 1u);
-            });
-            if (n_cand > batch) n_cand = batch;
-        }
     }
     for (uint32_t done = 0; done < n_cand; done += batch) {
     const uint32_t n_here = n_cand - done < batch ? n_cand - done : batch;
     blk.par([&](int tid) {
         if (static_cast<uint32_t>(tid) < batch)
             sm.word[tid] = static_cast<uint32_t>(tid) >= n_here ? 0ull : filtered ? sm.cand[done + tid]
-                           : surplus ? load_state(list + static_cast<long long>(dir) * static_cast<long long>(first + tid))   // written by another block
                            : list[static_cast<long long>(dir) * static_cast<long long>(first + tid)];   // dir = -1: a list that grows downwards
     });
     mark(16);
     arena_fill(blk, a, sm, ids, rk, batch, max_len);
     mark(17);
     // owner: a pre-token of 16 bytes or more that is itself in the vocabulary (ignore_merges)
-    if (!filtered && !surplus && tb.ignore_merges && max_len > static_cast<uint32_t>(kWordKeyMax)) {
+    if (!filtered && tb.ignore_merges && max_len > static_cast<uint32_t>(kWordKeyMax)) {
         blk.par([&](int tid) {
             if (static_cast<uint32_t>(tid) >= n_here) return;
             const unsigned long long wv = sm.word[tid];
@@ -3022,27 +2979,239 @@ GTOK_DEV void miss_batch(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsi
     }
 }
 
-// The two rare modes as functions of their own: inlined into the kernel beside the plain call they cost
-// every text a few percent of the kernel (registers and code size), used or not.
-template <class Blk>
-GTOK_DEV_NOINLINE void miss_batch_sharing(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsigned long long* list, int dir, uint32_t first, uint32_t n_miss,
-                                          uint32_t batch, uint32_t max_len, uint32_t take) {
-    miss_batch<Blk, 1>(blk, a, sm, list, dir, first, n_miss, batch, max_len, take);
-}
-template <class Blk>
-GTOK_DEV_NOINLINE void miss_batch_surplus(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsigned long long* list, int dir, uint32_t first, uint32_t n_miss) {
-    miss_batch<Blk, 2>(blk, a, sm, list, dir, first, n_miss, kMedBatchB, kMedSplit, kMedBatchB);
+// ---- kernel 3b: merging unknown pre-tokens of 2..64 bytes, several to a warp ----------
+// Greedy BPE (lowest rank first, leftmost among equals, src/host_encode.cc:617-648) applies one merge at a time, and the rules
+// for the two pairs that a merge makes are a dependent trip to L2 (0.6 us a step): a thread that walks the loop alone makes
+// up to 63 such trips in a row.  Here T lanes hold a pre-token of up to 4T bytes and apply in one round every merge that the
+// loop provably applies before it looks at anything this round does not know:
+//   * a pair whose key (rank << 6 | place) is below both neighbours' is `selected`; a pair beside a selected one with a lower
+//     key dies when that one is merged; the other pairs are `waiting`.
+//   * for each selected pair the rules for the two pairs that its merge would make are looked up, with a neighbour that is
+//     selected too and comes earlier already merged.  Let nu be the lower of their keys.
+//   * the loop takes the selected pairs in order of their keys until a new or a waiting pair is lower than the next of them.
+//     Selected pair s is therefore merged in this round exactly when key(s) <= the minimum of max(key(s'), nu(s')) over all
+//     selected s' and of the waiting pairs' keys.  (If key(s) is at most that, every s' before s has nu(s') >= key(s).  If
+//     not, the s' or waiting pair that gives the minimum stands in between.)  The lowest key always passes.
+// This asks nothing of the vocabulary (ranks need not be monotone).  On the multilingual text the longest of 32
+// pre-tokens of 49..64 bytes takes 9 rounds in place of 47 merges, of 17..32 bytes 7 in place of 24.
+// Four symbols a lane keep a warp full with 2, 4 or 8 pre-tokens, and every round packs the symbols left, so later rounds touch
+// fewer.  A round still costs several times the instructions of the merges it does, so this is the form for texts whose
+// pre-tokens the chip takes at once (use_teams).
+constexpr int kWarps = kThreads / 32;
+constexpr uint32_t kTeamSyms = 128;            // symbols of one warp's pre-tokens: 2 x 64, 4 x 32, 8 x 16
+constexpr uint32_t kTeamWords = 8 * kTeamSyms + kTeamSyms / 2;      // shared words of one warp
+static_assert(kWarps * kTeamWords <= 3 * kArenaSyms, "the warps' symbols fit the block's workspace");
+
+template <int T> struct TeamMask { typedef uint32_t type; };
+template <> struct TeamMask<16> { typedef uint64_t type; };
+GTOK_DEV uint32_t popc_mask(uint32_t x) { return static_cast<uint32_t>(popc32(x)); }
+GTOK_DEV uint32_t popc_mask(uint64_t x) { return static_cast<uint32_t>(popc32(static_cast<uint32_t>(x)) + popc32(static_cast<uint32_t>(x >> 32))); }
+
+// `entry(k)`: position | length << 32 of the warp's k-th pre-token (at most 4T bytes; 0 = none), k < 32 / T.
+// `ws`: kTeamWords words of shared memory of this warp's own.
+template <int T, class Warp, class Entry>
+GTOK_DEV void team_merge(Warp& wp, const EncodeArgs& a, const uint32_t* b2i, uint32_t* ws, Entry entry) {
+    typedef typename TeamMask<T>::type Mask;
+    constexpr uint32_t kMaxLen = 4 * T;
+    uint32_t* sym = ws;                             // symbols left, packed
+    uint32_t* key = ws + kTeamSyms;                 // of pair (i, i + 1): rank << 6 | i, kNoRank = no rule
+    uint32_t* res = ws + 2 * kTeamSyms;             // and the id it gives
+    uint32_t* other = ws + 3 * kTeamSyms;           // the three arrays of the next round
+    uint32_t* const nrank = ws + 6 * kTeamSyms;     // rules looked up in this round: at i the pair right of selected i, at i - 1 the one left of it
+    uint32_t* const nres = ws + 7 * kTeamSyms;
+    uint32_t* const list = ws + 8 * kTeamSyms;      // places of the selected pairs
+    struct Own { uint32_t g, n, e; Mask sel, com; };
+    typename Warp::template Local<Own> own;
+    typename Warp::template Local<uint32_t> flag;
+    wp.lanes([&](int lane) {
+        const uint32_t t = lane / T, q = lane % T, base = t * kMaxLen;
+        const unsigned long long wv = entry(t);
+        Own& o = own.at(lane);
+        o.g = static_cast<uint32_t>(wv);
+        o.n = static_cast<uint32_t>(wv >> 32);
+        uint32_t b[4];
+        GTOK_UNROLL
+        for (int it = 0; it < 4; ++it) b[it] = q + it * T < o.n ? ldg(a.text + o.g + q + it * T) : 0u;
+        GTOK_UNROLL
+        for (int it = 0; it < 4; ++it) if (q + it * T < o.n) sym[base + q + it * T] = b2i[b[it]];
+    });
+    wp.lanes([&](int lane) {
+        const uint32_t q = lane % T, base = lane / T * kMaxLen, n = own.at(lane).n;
+        GTOK_UNROLL
+        for (int it = 0; it < 4; it += 2) {
+            const uint32_t i = q + it * T, j = i + T;
+            const bool wi = i + 1 < n, wj = j + 1 < n;
+            RankRes x, y;
+            probe_rule2(a.tb, wi, wi ? sym[base + i] : 0u, wi ? sym[base + i + 1] : 0u, &x, wj, wj ? sym[base + j] : 0u, wj ? sym[base + j + 1] : 0u, &y);
+            if (i < n) { key[base + i] = rank_key(x.rank, i); res[base + i] = x.res; }
+            if (j < n) { key[base + j] = rank_key(y.rank, j); res[base + j] = y.res; }
+        }
+    });
+    for (;;) {
+        wp.lanes_nosync([&](int lane) { flag.at(lane) = own.at(lane).n; });
+        const uint32_t its = (wp.max(flag) + T - 1u) / T;           // symbols a lane holds of the longest pre-token left: 4, then fewer
+        wp.lanes([&](int lane) { own.at(lane).sel = 0; own.at(lane).com = 0; own.at(lane).e = kNoRank; });
+        uint32_t any = 0;
+        for (uint32_t it = 0; it < its; ++it) {
+            wp.lanes_nosync([&](int lane) {
+                const uint32_t i = lane % T + it * T, base = lane / T * kMaxLen, n = own.at(lane).n;
+                uint32_t s = 0;
+                if (i + 1 < n) {
+                    const uint32_t k = key[base + i], kl = i ? key[base + i - 1] : kNoRank, kr = key[base + i + 1];     // (the last symbol's is kNoRank)
+                    s = k < kl && k < kr;
+                }
+                flag.at(lane) = s;
+            });
+            const uint32_t b = wp.ballot(flag);
+            any |= b;
+            wp.lanes_nosync([&](int lane) { own.at(lane).sel |= static_cast<Mask>((b >> (lane / T * T)) & ((1u << T) - 1u)) << (it * T); });
+        }
+        if (!any) break;
+        wp.lanes([&](int lane) {
+            const Mask sel = own.at(lane).sel;
+            uint32_t* const l = list + lane / T * (kMaxLen / 2);
+            for (uint32_t it = 0; it < its; ++it) {
+                const uint32_t i = lane % T + it * T;
+                if ((sel >> i) & 1u) l[popc_mask(static_cast<Mask>(sel & ((static_cast<Mask>(1) << i) - 1u)))] = i;
+            }
+        });
+        // what their merges would make
+        for (uint32_t c0 = 0;; c0 += T) {
+            wp.lanes_nosync([&](int lane) { flag.at(lane) = c0 < popc_mask(own.at(lane).sel); });
+            if (!wp.ballot(flag)) break;
+            wp.lanes_nosync([&](int lane) {
+                Own& o = own.at(lane);
+                const uint32_t c = c0 + lane % T, base = lane / T * kMaxLen;
+                if (c >= popc_mask(o.sel)) return;
+                const uint32_t i = list[lane / T * (kMaxLen / 2) + c], x = base + i;
+                const uint32_t k = key[x], merged = res[x];
+                const bool hr = i + 2 < o.n, hl = i != 0;
+                const uint32_t rs = hr ? (((o.sel >> (i + 2)) & 1u) && key[x + 2] < k ? res[x + 2] : sym[x + 2]) : 0u;
+                const uint32_t ls = hl ? (i >= 2 && ((o.sel >> (i - 2)) & 1u) && key[x - 2] < k ? res[x - 2] : sym[x - 1]) : 0u;
+                RankRes right, left;
+                probe_rule2(a.tb, hr, merged, rs, &right, hl, ls, merged, &left);
+                nrank[x] = right.rank; nres[x] = right.res;
+                if (hl) { nrank[x - 1] = left.rank; nres[x - 1] = left.res; }
+                const uint32_t kr = rank_key(right.rank, i), kl = hl ? rank_key(left.rank, i - 1) : kNoRank;
+                const uint32_t nu = kl < kr ? kl : kr, e = nu > k ? nu : k;
+                if (e < o.e) o.e = e;
+            });
+        }
+        // the bound, and who passes it
+        wp.lanes([&](int lane) {
+            Own& o = own.at(lane);
+            const Mask near = o.sel | static_cast<Mask>(o.sel << 1) | (o.sel >> 1);
+            const uint32_t base = lane / T * kMaxLen;
+            for (uint32_t it = 0; it < its; ++it) {
+                const uint32_t i = lane % T + it * T;
+                if (i + 1 < o.n && !((near >> i) & 1u)) { const uint32_t k = key[base + i]; if (k < o.e) o.e = k; }
+            }
+            flag.at(lane) = o.e;
+        });
+        wp.template team_min<T>(flag);
+        wp.lanes_nosync([&](int lane) { own.at(lane).e = flag.at(lane); });
+        for (uint32_t it = 0; it < its; ++it) {
+            wp.lanes_nosync([&](int lane) {
+                const Own& o = own.at(lane);
+                const uint32_t i = lane % T + it * T;
+                flag.at(lane) = ((o.sel >> i) & 1u) && key[lane / T * kMaxLen + i] <= o.e;
+            });
+            const uint32_t b = wp.ballot(flag);
+            wp.lanes_nosync([&](int lane) { own.at(lane).com |= static_cast<Mask>((b >> (lane / T * T)) & ((1u << T) - 1u)) << (it * T); });
+        }
+        // the symbols left, each with the rule of the pair it now opens, packed
+        wp.lanes([&](int lane) {
+            Own& o = own.at(lane);
+            const uint32_t base = lane / T * kMaxLen;
+            for (uint32_t it = 0; it < its; ++it) {
+                const uint32_t i = lane % T + it * T, x = base + i;
+                if (i >= o.n || ((static_cast<Mask>(o.com << 1) >> i) & 1u)) continue;           // none there, or merged into the one before
+                const uint32_t com = static_cast<uint32_t>(o.com >> i) & 1u, v = i + 1u + com;    // v: the symbol after it
+                const uint32_t at = i - popc_mask(static_cast<Mask>(o.com & ((static_cast<Mask>(1) << i) - 1u)));
+                const uint32_t kx = key[x];
+                uint32_t k = kx == kNoRank ? kNoRank : kx >> 6, r = res[x];
+                other[base + at] = com ? r : sym[x];
+                if (v >= o.n) k = kNoRank;
+                else {
+                    const bool vc = (o.com >> v) & 1u;
+                    if (vc && !(com && kx > key[base + v])) { k = nrank[base + v - 1]; r = nres[base + v - 1]; }     // the later of the two merges looked this pair up
+                    else if (com) { k = nrank[x]; r = nres[x]; }
+                }
+                other[kTeamSyms + base + at] = rank_key(k, at);
+                other[2 * kTeamSyms + base + at] = r;
+            }
+            o.n -= popc_mask(o.com);
+        });
+        uint32_t* const was = sym;
+        sym = other; key = other + kTeamSyms; res = other + 2 * kTeamSyms;
+        other = was;
+    }
+    wp.lanes([&](int lane) {
+        const Own& o = own.at(lane);
+        const uint32_t q = lane % T, base = lane / T * kMaxLen;
+        GTOK_UNROLL
+        for (int it = 0; it < 4; ++it) if (q + it * T < o.n) put_id(a, o.g, q + it * T, sym[base + q + it * T]);
+        if (q == 0 && o.n) global_add(a.tile_tok + o.g / kTile, o.n);
+    });
 }
 
-// What a call of the 17..32-byte class with `share` left behind: chunk `chunk` of the surplus of the
-// call that began at list entry `first`.  The entries are known not to be vocabulary tokens.
-constexpr uint32_t kSurplusChunks = (kMedTakeB - kMedBatchB + kMedBatchB - 1) / kMedBatchB;
+// One call of this form: `take` entries (at most kThreads) from entry `first` on of a list of pre-tokens of at most `max_len`
+// bytes (dir = -1: a list that grows downwards).  Under ignore_merges a pre-token of more than kWordKeyMax bytes that is itself
+// a vocabulary token is found first, a thread each; the warps merge the rest, each on its own.
 template <class Blk>
-GTOK_DEV void miss_surplus(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsigned long long* list, int dir, uint32_t first, uint32_t chunk) {
-    const uint32_t extra = static_cast<uint32_t>(load_state(list + static_cast<long long>(dir) * static_cast<long long>(first)));
-    if (chunk * kMedBatchB >= extra) return;
-    miss_batch_surplus(blk, a, sm, list, dir, first + 1u + chunk * kMedBatchB, first + 1u + extra);
+GTOK_DEV void miss_teams(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsigned long long* list, int dir, uint32_t first, uint32_t n_list,
+                         uint32_t take, uint32_t max_len) {
+    const DeviceTables& tb = a.tb;
+    const uint32_t n_take = n_list - first < take ? n_list - first : take;
+    uint32_t n_cand = n_take;
+    blk.par([&](int tid) {
+        if (tid == 0) sm.ctr[C_USED] = 0;
+        if (static_cast<uint32_t>(tid) < n_take) sm.cand[tid] = list[static_cast<long long>(dir) * static_cast<long long>(first + tid)];
+    });
+    if (tb.ignore_merges && max_len > static_cast<uint32_t>(kWordKeyMax)) {
+        uint8_t* stage_bytes = reinterpret_cast<uint8_t*>(sm.ws);        // the entries' bytes, max_len apart
+        stage_entries(blk, a, sm.cand, n_take, max_len, stage_bytes);
+        typename Blk::template Local<unsigned long long> left;
+        blk.par([&](int tid) {
+            left.at(tid) = 0ull;
+            if (static_cast<uint32_t>(tid) >= n_take) return;
+            const unsigned long long wv = sm.cand[tid];
+            const uint32_t g = static_cast<uint32_t>(wv), len = static_cast<uint32_t>(wv >> 32);
+            const uint32_t id = len <= static_cast<uint32_t>(kWordKeyMax) ? kNoToken : probe_long_bytes(tb, stage_bytes + tid * max_len, len);
+            if (id != kNoToken) { put_id(a, g, 0, id); global_add(a.tile_tok + g / kTile, 1u); }
+            else left.at(tid) = wv;
+        });
+        blk.par([&](int tid) {
+            const unsigned long long wv = left.at(tid);
+            if (wv) sm.cand[shared_add(&sm.ctr[C_USED], 1u)] = wv;
+        });
+        n_cand = sm.ctr[C_USED];
+    }
+    blk.warps([&](auto& wp) {
+        uint32_t* ws = sm.ws + wp.index * kTeamWords;
+        auto run = [&](auto team) {
+            constexpr int T = decltype(team)::value;
+            constexpr uint32_t kEach = 32 / T;
+            for (uint32_t w0 = wp.index * kEach; w0 < n_cand; w0 += kWarps * kEach)
+                team_merge<T>(wp, a, sm.b2i, ws, [&](uint32_t k) { return w0 + k < n_cand ? sm.cand[w0 + k] : 0ull; });
+        };
+        if (max_len > static_cast<uint32_t>(kMedSplit)) run(std::integral_constant<int, 16>());
+        else if (max_len > static_cast<uint32_t>(kShortWordMax)) run(std::integral_constant<int, 8>());
+        else run(std::integral_constant<int, 4>());
+    });
 }
+
+// Entries per call: what the block's warps hold at once (16, 32 or 64; the length class decides).
+GTOK_DEV uint32_t team_take(uint32_t max_len) {
+    return (max_len > static_cast<uint32_t>(kMedSplit) ? 2u : max_len > static_cast<uint32_t>(kShortWordMax) ? 4u : 8u) * kWarps;
+}
+// Whether a text's pre-tokens of 17..64 bytes are merged by teams: while they make at most one call a block, the kernel lasts as
+// long as one call and the chain counts; beyond, instructions do.  Merge kernel, teams / one thread a pre-token (592 blocks):
+// multilingual text of 0.1 MB 34 / 58 us, 1.2 MB 44 / 65, 2.4 MB (some 550 calls) 63 / 67, 4.5 MB 97 / 69; code and CJK
+// 0.1 MB 30 / 60, 1.2 MB (660 calls) 50 / 67, 2.4 MB 75 / 69; adversarial text 0.4 MB 54 / 91, 4.5 MB (650 calls) 93 / 106,
+// 8 MB 159 / 122.  Pre-tokens of up to 16 bytes have short chains: one thread each is as fast at every size (English, 0.1 to
+// 8 MB: 24 / 24 to 50 / 52; by teams 27 to 84), but in the single-block kernel, where all lengths share one list.
+GTOK_DEV bool use_teams(uint32_t calls, uint32_t blocks) { return calls <= blocks; }
 
 // ---- run-length path for long pre-tokens made of a few byte runs ------------------------
 // A very long pre-token is, in practice, a run of one character (spaces, newlines, dashes,

@@ -120,22 +120,12 @@ __global__ void __launch_bounds__(kThreads, 4) miss_kernel(const __grid_constant
     __shared__ uint32_t s_pick;
     GpuBlk blk;
     const uint32_t n_miss = a.ctl[CTL_NMISS], n_med = a.ctl[CTL_NMED], n_med1 = a.ctl[CTL_NMED1], n_med2 = a.ctl[CTL_NMED2], n_long = a.ctl[CTL_NLONG];
-    const uint32_t take_b = a.tb.ignore_merges ? kMedTakeB : kMedBatchB;      // list entries per call of the 17..32-byte class
-    const uint32_t med2_batches = (n_med2 + take_b - 1) / take_b;
-    const uint32_t short_batches = (n_miss + kMissBatch - 1) / kMissBatch;
-    // Pre-tokens per call of the two longest classes: an arena's worth, unless that leaves most blocks without a call (a
-    // prompt, a shard of a document): then a quarter, so that a call's fetch and pair phases, which the merge chains wait for,
-    // are a quarter as long.
-    uint32_t batch_a = kMedBatchA, batch_a1 = kMedBatchA1;
-    if (2u * ((n_med + kMedBatchA / 4 - 1) / (kMedBatchA / 4) + (n_med1 + kMedBatchA1 / 4 - 1) / (kMedBatchA1 / 4) + med2_batches + short_batches + n_long) < gridDim.x) {
-        batch_a = kMedBatchA / 4;
-        batch_a1 = kMedBatchA1 / 4;
-    }
-    const uint32_t med_batches = (n_med + batch_a - 1) / batch_a, med1_batches = (n_med1 + batch_a1 - 1) / batch_a1;
-    // A call of the 17..32-byte class under ignore_merges looks 256 entries up as whole tokens but merges at most 96
-    // of them at a time.  With fewer calls than blocks (a prompt rather than a corpus) it hands the rest back for the
-    // blocks that got no call; otherwise it works through the rest itself, which keeps the blocks evenly loaded.
-    const bool share = take_b > kMedBatchB && med2_batches != 0 && med_batches + med1_batches + med2_batches + short_batches + n_long < gridDim.x;
+    auto calls = [](uint32_t n, uint32_t take) { return (n + take - 1) / take; };
+    // Which form merges them (use_teams), and the entries per call of each class
+    const bool teams = use_teams(calls(n_med, team_take(kMedWordMax)) + calls(n_med1, team_take(kMedWordMax)) + calls(n_med2, team_take(kMedSplit)), gridDim.x);
+    const uint32_t take_a = teams ? team_take(kMedWordMax) : kMedBatchA, take_a1 = teams ? team_take(kMedWordMax) : kMedBatchA1;
+    const uint32_t take_b = teams ? team_take(kMedSplit) : a.tb.ignore_merges ? kMedTakeB : kMedBatchB;
+    const uint32_t med_calls = calls(n_med, take_a), med1_calls = calls(n_med1, take_a1), med2_calls = calls(n_med2, take_b), short_calls = calls(n_miss, kMissBatch);
     tl_stamp(a, 2, 0);
     sm.b2i[threadIdx.x] = a.tb.byte_to_id[threadIdx.x];
     __syncthreads();
@@ -154,36 +144,18 @@ __global__ void __launch_bounds__(kThreads, 4) miss_kernel(const __grid_constant
         __syncthreads();
         const uint32_t t = s_pick;
         __syncthreads();
-        if (t >= med_batches + med1_batches + med2_batches + short_batches) break;
+        if (t >= med_calls + med1_calls + med2_calls + short_calls) break;
         const unsigned long long* list = a.gmiss;
         int dir = 1;
-        uint32_t first = (t - med_batches - med1_batches - med2_batches) * kMissBatch, count = n_miss, batch = kMissBatch, max_len = kShortWordMax, take = kMissBatch;
-        if (t < med_batches) { list = a.gmed; first = t * batch_a; count = n_med; batch = batch_a; max_len = kMedWordMax; take = batch_a; }
-        else if (t < med_batches + med1_batches) { list = a.gmed1; first = (t - med_batches) * batch_a1; count = n_med1; batch = batch_a1; max_len = kMedSplit1; take = batch_a1; }
-        else if (t < med_batches + med1_batches + med2_batches) {
-            list = a.gmed + (a.gmed_cap - 1); dir = -1; first = (t - med_batches - med1_batches) * take_b; count = n_med2; batch = kMedBatchB; max_len = kMedSplit; take = take_b;
+        uint32_t first = (t - med_calls - med1_calls - med2_calls) * kMissBatch, count = n_miss, batch = kMissBatch, max_len = kShortWordMax, take = kMissBatch;
+        if (t < med_calls) { list = a.gmed; first = t * take_a; count = n_med; batch = kMedBatchA; max_len = kMedWordMax; take = take_a; }
+        else if (t < med_calls + med1_calls) { list = a.gmed1; first = (t - med_calls) * take_a1; count = n_med1; batch = kMedBatchA1; max_len = kMedSplit1; take = take_a1; }
+        else if (t < med_calls + med1_calls + med2_calls) {
+            list = a.gmed + (a.gmed_cap - 1); dir = -1; first = (t - med_calls - med1_calls) * take_b; count = n_med2; batch = kMedBatchB; max_len = kMedSplit; take = take_b;
         }
-        if (share && take > batch) miss_batch_sharing(blk, a, sm, list, dir, first, count, batch, max_len, take);
+        if (teams && t < med_calls + med1_calls + med2_calls) miss_teams(blk, a, sm, list, dir, first, count, take, max_len);
         else miss_batch(blk, a, sm, list, dir, first, count, batch, max_len, take);
         tl_stamp(a, 2, 2 + done);
-    }
-    // What the calls of the 17..32-byte class handed back: wait until every such call is through its lookups, then
-    // take the chunks in turn.  The wait is for blocks that are running (a call is only ever held by a block that
-    // took its ticket).
-    if (share) {
-        if (threadIdx.x == 0)
-            s_pick = wait_count(a.ctl + CTL_FILTERED, med2_batches, a.ctl) && *reinterpret_cast<volatile uint32_t*>(a.ctl + CTL_NSURPLUS) ? 1u : 0u;   // usually nothing
-        __syncthreads();
-        const bool ready = s_pick != 0;
-        __syncthreads();
-        while (ready) {
-            if (threadIdx.x == 0) s_pick = atomicAdd(a.ctl + CTL_SURPLUS, 1u);
-            __syncthreads();
-            const uint32_t u = s_pick;
-            __syncthreads();
-            if (u >= med2_batches * kSurplusChunks) break;
-            miss_surplus(blk, a, sm, a.gmed + (a.gmed_cap - 1), -1, (u / kSurplusChunks) * take_b, u % kSurplusChunks);
-        }
     }
     tl_stamp(a, 2, 1);
 }

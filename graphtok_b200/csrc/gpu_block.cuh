@@ -21,6 +21,37 @@ struct GpuBlk {
         f(static_cast<int>(threadIdx.x));
         __syncthreads();
     }
+    // One of the block's warps, which then run on their own up to the barrier at the end.
+    struct Warp {
+        int index;
+        template <class T>
+        struct Local {
+            T v;
+            __device__ __forceinline__ T& at(int) { return v; }
+        };
+        template <class F>
+        __device__ __forceinline__ void lanes(F f) {
+            f(static_cast<int>(threadIdx.x & 31u));
+            __syncwarp();
+        }
+        // for steps that leave nothing in shared memory that another lane reads before the next lanes()
+        template <class F>
+        __device__ __forceinline__ void lanes_nosync(F f) { f(static_cast<int>(threadIdx.x & 31u)); }
+        __device__ __forceinline__ uint32_t ballot(Local<uint32_t>& x) { return __ballot_sync(0xFFFFFFFFu, x.v != 0); }
+        __device__ __forceinline__ uint32_t max(Local<uint32_t>& x) { return __reduce_max_sync(0xFFFFFFFFu, x.v); }
+        // every lane gets the lowest value of its group of T lanes
+        template <int T>
+        __device__ __forceinline__ void team_min(Local<uint32_t>& x) {
+#pragma unroll
+            for (int d = T / 2; d; d >>= 1) x.v = ::min(x.v, __shfl_xor_sync(0xFFFFFFFFu, x.v, d));
+        }
+    };
+    template <class F>
+    __device__ __forceinline__ void warps(F f) {
+        Warp wp{static_cast<int>(threadIdx.x >> 5)};
+        f(wp);
+        __syncthreads();
+    }
     // In-place exclusive scan of arr[kThreads] (shared memory); every thread gets the total.
     __device__ __forceinline__ void excl_scan(uint32_t* arr, uint32_t* total) {
         __shared__ uint32_t wsum[kThreads / 32];

@@ -73,8 +73,9 @@ __global__ void __launch_bounds__(kThreads, 1) tiny_kernel(const __grid_constant
     tl_stamp(a, 5, 3);
     {
         MissSmem& ms = sm.miss;
-        // every unknown pre-token of 2..64 bytes is in the one list (a.one_list): batches as large as the
-        // longest of them allows, so that a short prompt's merge loops all run side by side
+        // every unknown pre-token of 2..64 bytes is in the one list (a.one_list): teams as wide as the longest of them needs, so
+        // that a short prompt's merge loops all run side by side (951 bytes in a script other than Latin: 72 us a call with
+        // one thread a pre-token, 59 with teams)
         const uint32_t n_miss = a.ctl[CTL_NMISS], n_long = a.ctl[CTL_NLONG];
         __shared__ uint32_t s_maxlen;
         if (tid == 0) s_maxlen = 0;
@@ -87,13 +88,8 @@ __global__ void __launch_bounds__(kThreads, 1) tiny_kernel(const __grid_constant
         }
         __syncthreads();
         const uint32_t longest = s_maxlen;
-        uint32_t batch = kMissBatch, max_len = kShortWordMax;
-        if (longest > static_cast<uint32_t>(kMedSplit1)) { batch = kMedBatchA; max_len = kMedWordMax; }
-        else if (longest > static_cast<uint32_t>(kMedSplit)) { batch = kMedBatchA1; max_len = kMedSplit1; }
-        else if (longest > static_cast<uint32_t>(kShortWordMax)) { batch = kMedBatchB; max_len = kMedSplit; }
-        // (no more arena than there are entries: the fetch and pair phases pass over batch * max_len slots)
-        if (n_miss < batch) batch = n_miss ? (n_miss + 3u) & ~3u : 4u;
-        for (uint32_t first = 0; first < n_miss; first += batch) miss_batch(blk, a, ms, a.gmiss, 1, first, n_miss, batch, max_len, batch);
+        const uint32_t max_len = longest > static_cast<uint32_t>(kMedSplit) ? kMedWordMax : longest > static_cast<uint32_t>(kShortWordMax) ? kMedSplit : kShortWordMax;
+        for (uint32_t first = 0; first < n_miss; first += kThreads) miss_teams(blk, a, ms, a.gmiss, 1, first, n_miss, kThreads, max_len);
         for (uint32_t li = 0; li < n_long; ++li) long_word(blk, a, ms, li);
     }
     __syncthreads();

@@ -95,7 +95,7 @@ def tile_crossers(special):
     for alphabet, length in (("abcdefghijklmnopqrstuvwxyz", 20000), ("ACGT", 9000), ("etaoinshr", 3000), ("ab", 700), ("theinandofto", 5000),
                              ("中文日本語的一是不了人我在有他这为之大来以个", 2500), ("éèêàùç", 900), ("!@#$%^&*()-=+", 4000)):
         out.append("p " + "".join(rng.choice(alphabet) for _ in range(length)) + " q")
-    # many pre-tokens of 17 to 32 bytes that are no vocabulary tokens (what one block does not merge itself it hands back),
+    # many pre-tokens of 17 to 32 bytes that are no vocabulary tokens (several arenas to a call),
     # alone and among ones that may be
     b64 = "ABCDEFGHIJKLMNOPQRSTUVWXYZabcdefghijklmnopqrstuvwxyz0123456789+/"
     out.append(" ".join("".join(rng.choice(b64[:52]) for _ in range(rng.randint(17, 32))) for _ in range(900)))

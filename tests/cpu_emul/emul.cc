@@ -35,6 +35,46 @@ struct CpuBlk {
         if (!reverse) for (int t = 0; t < gtok::kThreads; ++t) f(t);
         else for (int t = gtok::kThreads - 1; t >= 0; --t) f(t);
     }
+    // One of the block's warps: its lanes one after the other, in the same direction as the threads.
+    struct Warp {
+        int index;
+        bool reverse;
+        template <class T>
+        struct Local {
+            T v[32];
+            T& at(int lane) { return v[lane]; }
+        };
+        template <class F> void lanes(F f) {
+            if (!reverse) for (int t = 0; t < 32; ++t) f(t);
+            else for (int t = 31; t >= 0; --t) f(t);
+        }
+        template <class F> void lanes_nosync(F f) { lanes(f); }
+        uint32_t ballot(Local<uint32_t>& x) {
+            uint32_t b = 0;
+            for (int t = 0; t < 32; ++t) b |= (x.v[t] ? 1u : 0u) << t;
+            return b;
+        }
+        uint32_t max(Local<uint32_t>& x) {
+            uint32_t m = 0;
+            for (int t = 0; t < 32; ++t) if (x.v[t] > m) m = x.v[t];
+            return m;
+        }
+        template <int T> void team_min(Local<uint32_t>& x) {
+            for (int t = 0; t < 32; t += T) {
+                uint32_t m = 0xFFFFFFFFu;
+                for (int i = t; i < t + T; ++i) if (x.v[i] < m) m = x.v[i];
+                for (int i = t; i < t + T; ++i) x.v[i] = m;
+            }
+        }
+    };
+    template <class F> void warps(F f) {
+        for (int k = 0; k < gtok::kThreads / 32; ++k) {
+            Warp wp;
+            wp.index = reverse ? gtok::kThreads / 32 - 1 - k : k;
+            wp.reverse = reverse;
+            f(wp);
+        }
+    }
     void excl_scan(uint32_t* arr, uint32_t* total) {
         uint32_t acc = 0;
         for (int i = 0; i < gtok::kThreads; ++i) { uint32_t v = arr[i]; arr[i] = acc; acc += v; }
@@ -174,17 +214,18 @@ int64_t gtok_emul_encode(void* h, const uint8_t* text, uint32_t n, const uint32_
         std::memset(sm, 0xCD, sizeof *sm);
         for (int i = 0; i < 256; ++i) sm->b2i[i] = a.tb.byte_to_id[i];
         const uint32_t n_miss = ctl[CTL_NMISS], n_med = ctl[CTL_NMED], n_med1 = ctl[CTL_NMED1], n_med2 = ctl[CTL_NMED2], n_long = ctl[CTL_NLONG];
-        for (uint32_t first = 0; first < n_med; first += kMedBatchA) miss_batch(blk, a, *sm, a.gmed, 1, first, n_med, kMedBatchA, kMedWordMax, kMedBatchA);
-        for (uint32_t first = 0; first < n_med1; first += kMedBatchA1) miss_batch(blk, a, *sm, a.gmed1, 1, first, n_med1, kMedBatchA1, kMedSplit1, kMedBatchA1);
-        const uint32_t take_b = a.tb.ignore_merges ? kMedTakeB : kMedBatchB;
-        for (uint32_t first = 0; first < n_med2; first += take_b) {
-            if (take_b > kMedBatchB) miss_batch_sharing(blk, a, *sm, a.gmed + (a.gmed_cap - 1), -1, first, n_med2, kMedBatchB, kMedSplit, take_b);
-            else miss_batch(blk, a, *sm, a.gmed + (a.gmed_cap - 1), -1, first, n_med2, kMedBatchB, kMedSplit, take_b);
-        }
-        if (take_b > kMedBatchB)
-            for (uint32_t first = 0; first < n_med2; first += take_b)
-                for (uint32_t c = 0; c < kSurplusChunks; ++c) miss_surplus(blk, a, *sm, a.gmed + (a.gmed_cap - 1), -1, first, c);
-        for (uint32_t first = 0; first < n_miss; first += kMissBatch) miss_batch(blk, a, *sm, a.gmiss, 1, first, n_miss, kMissBatch, kShortWordMax, kMissBatch);
+        // (the runs in order merge by teams, the reversed ones a thread a pre-token, whatever the size; the kernel takes one or the other by size)
+        auto merge = [&](const unsigned long long* list, int dir, uint32_t count, uint32_t batch, uint32_t max_len, uint32_t take) {
+            if (!reverse) take = team_take(max_len);
+            for (uint32_t first = 0; first < count; first += take) {
+                if (reverse) miss_batch(blk, a, *sm, list, dir, first, count, batch, max_len, take);
+                else miss_teams(blk, a, *sm, list, dir, first, count, take, max_len);
+            }
+        };
+        merge(a.gmed, 1, n_med, kMedBatchA, kMedWordMax, kMedBatchA);
+        merge(a.gmed1, 1, n_med1, kMedBatchA1, kMedSplit1, kMedBatchA1);
+        merge(a.gmed + (a.gmed_cap - 1), -1, n_med2, kMedBatchB, kMedSplit, a.tb.ignore_merges ? kMedTakeB : kMedBatchB);
+        merge(a.gmiss, 1, n_miss, kMissBatch, kShortWordMax, kMissBatch);
         for (uint32_t li = 0; li < n_long; ++li) long_word(blk, a, *sm, li);
         delete sm;
     }
