@@ -513,13 +513,31 @@ struct PretokSmem {
 // With the wide class table (DeepSeek-V3) the block's copy of the narrow table is not used, and its
 // room holds four more planes: punctuation and symbols, ASCII letters, ASCII punctuation, and the lead
 // bytes of codepoints inside the three CJK ranges.
-enum { XP_PS = 0, XP_AL, XP_APU, XP_CJK, kXPlanes };
+// (Gemma-3 shape: characters a rule may join to a U+2581 after them in XP_PS, and in the others the bytes from 0xC0, 0xE0
+// and 0xF0 on, which give a whole character's width.)
+enum { XP_PS = 0, XP_AL, XP_APU, XP_CJK, kXPlanes, XP_W2 = XP_AL, XP_W3 = XP_APU, XP_W4 = XP_CJK };
 constexpr int kXPlaneStride = kPWin / 16 + 8;
 static_assert(kXPlanes * kXPlaneStride * 2 <= kUcStage2Words * 4, "the extra planes fit the class-table copy");
 GTOK_DEV uint16_t* xplane(PretokSmem& sm, int k) { return reinterpret_cast<uint16_t*>(sm.ucs2) + k * kXPlaneStride; }
 GTOK_DEV const uint16_t* xplane(const PretokSmem& sm, int k) { return reinterpret_cast<const uint16_t*>(sm.ucs2) + k * kXPlaneStride; }
 // Their entries of chunk c from its attribute bytes and its text.
-GTOK_DEV void chunk_xplanes(PretokSmem& sm, int c, const uint32_t* aw, const uint32_t* tw) {
+GTOK_DEV void chunk_xplanes(PretokSmem& sm, int c, const uint32_t* aw, const uint32_t* tw, bool chars) {
+    if (chars) {
+        uint32_t p6 = 0, w2 = 0, w3 = 0, w4 = 0;
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t x = (aw[j] & 0x07070707u) ^ (A_P * 0x01010101u), t = tw[j];
+            p6 |= gather_bit4(~(((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u, 7) << (4 * j);
+            const uint32_t t2 = t & (t << 1), t3 = t2 & (t << 2), t4 = t3 & (t << 3);      // (a byte's own bits only reach its top bit)
+            w2 |= gather_bit4(t2, 7) << (4 * j);
+            w3 |= gather_bit4(t3, 7) << (4 * j);
+            w4 |= gather_bit4(t4, 7) << (4 * j);
+        }
+        xplane(sm, XP_PS)[c] = static_cast<uint16_t>(p6);
+        xplane(sm, XP_W2)[c] = static_cast<uint16_t>(w2);
+        xplane(sm, XP_W3)[c] = static_cast<uint16_t>(w3);
+        xplane(sm, XP_W4)[c] = static_cast<uint16_t>(w4);
+        return;
+    }
     uint32_t ps = 0, al = 0, asc = 0, cjk = 0;
     for (int j = 0; j < 4; ++j) {
         const uint32_t x = (aw[j] & 0x07070707u) ^ (A_P * 0x01010101u);            // a zero byte: class A_P
@@ -1152,73 +1170,6 @@ GTOK_DEV bool ds_mark_takes_letters(const Win& w, int m, uint8_t am) {
     if (q < 0) return true;
     return !((aq & A_CLS) == A_P || (aq & A_SP));
 }
-// ---- Gemma-3 shape ----
-// The model merges the characters of the whole text, so any cut must be one that no rule can reach across.  Two
-// kinds are taken.  A byte that is not part of a whole character of the vocabulary (a character the vocabulary lacks,
-// malformed UTF-8, a character cut by a document's end) stands alone: the model spells it as its "<0xNN>" token,
-// which no rule mentions, and keeping such bytes apart is also what keeps the loader's byte-to-character rules from
-// ever seeing them.  And a space (U+0020, which the normaliser writes as U+2581, or that character itself) opens a
-// pre-token unless some rule's left side ends with the character before it while its right side begins with U+2581
-// (class 6 in the vocabulary's class table; 0 any other character of the vocabulary, 3 everything else).
-// Every byte of the tile is decided here, by strict decoding of the bytes around it.
-GTOK_DEV bool sp_docstart_at(const Win& w, int p) {
-    const int i = p - w.lo;
-    if (i >= 0 && i < kPWin) return (w.sm->dsw[i >> 5] >> (i & 31)) & 1u;
-    return is_docstart_global(*w.a, p);
-}
-// The whole character that holds byte p, inside p's document: its first byte in *start, its codepoint in *cp; 0 when
-// there is none, else its width.
-GTOK_DEV int sp_char_at(const Win& w, int p, int* start, uint32_t* cp) {
-    int s = p;
-    for (int k = 0; (text_at(w, s) & 0xC0u) == 0x80u; ++k) {
-        if (k == 3 || s == 0 || sp_docstart_at(w, s)) return 0;
-        --s;
-    }
-    const uint32_t b0 = text_at(w, s);
-    int width;
-    if (b0 < 0x80u) width = 1;
-    else if (b0 >= 0xC2u && b0 <= 0xDFu) width = 2;
-    else if (b0 >= 0xE0u && b0 <= 0xEFu) width = 3;
-    else if (b0 >= 0xF0u && b0 <= 0xF4u) width = 4;
-    else return 0;
-    if (s + width > w.n || p >= s + width) return 0;
-    uint32_t v = width == 1 ? b0 : width == 2 ? (b0 & 0x1Fu) : width == 3 ? (b0 & 0x0Fu) : (b0 & 0x07u);
-    for (int k = 1; k < width; ++k) {
-        const uint32_t b = text_at(w, s + k);
-        if ((b & 0xC0u) != 0x80u || sp_docstart_at(w, s + k)) return 0;
-        v = (v << 6) | (b & 0x3Fu);
-    }
-    if ((width == 3 && (v < 0x800u || (v >= 0xD800u && v <= 0xDFFFu))) || (width == 4 && (v < 0x10000u || v > 0x10FFFFu))) return 0;
-    *start = s;
-    *cp = v;
-    return width;
-}
-// Class of the whole character cp that begins at s.  Inside the window the classification phase has looked it up already
-// (a well-formed sequence decodes there to the same codepoint); outside, from the table in global memory.
-GTOK_DEV uint32_t sp_class(const Win& w, int s, uint32_t cp) {
-    if (s >= w.vlo && s < w.vhi) {
-        const uint32_t k = w.sm->attr[s - w.lo] & A_CLS;
-        if (k == 0u || k == 3u || k == 6u) return k;              // (an added token's bytes carry another class: the long way then)
-    }
-    const EncodeArgs& a = *w.a;
-    return uc_class([&](uint32_t i) { return static_cast<uint32_t>(ldg(a.tb.uc_stage1 + i)); }, [&](uint32_t i) { return ldg(a.tb.uc_stage2 + i); }, cp, true);
-}
-GTOK_DEV_NOINLINE bool is_boundary_sp(const Win& w, int p) {
-    if (p == 0 || sp_docstart_at(w, p)) return true;
-    int s = 0, s1 = 0;
-    uint32_t cp = 0, c1 = 0;
-    if (!sp_char_at(w, p, &s, &cp) || sp_class(w, s, cp) == 3u) return true;       // on its own, byte by byte
-    if (s != p) return false;                                                         // inside a character
-    // what ends right before p: an added token, a byte on its own, or a character
-    const int q = prev_lead(w, p);
-    if (q < 0 || (attr_at(w, q) & A_CLS) == A_ADDED) return true;
-    if (!sp_char_at(w, p - 1, &s1, &c1)) return true;
-    const uint32_t k1 = sp_class(w, s1, c1);
-    if (k1 == 3u) return true;
-    if (cp == 0x20u || cp == 0x2581u) return k1 != 6u;
-    return false;
-}
-
 GTOK_DEV_NOINLINE bool is_boundary_deepseek(const Win& w, int p, uint8_t a0, bool* pending, bool* nstart) {
     *pending = false;
     const int cur = a0 & A_CLS;
@@ -1748,6 +1699,16 @@ GTOK_DEV void pretok_tile(Blk& blk, const EncodeArgs& a, PretokSmem& sm, int til
                     if (kWide) {
                         cls = uc_class([&](uint32_t k) { return static_cast<uint32_t>(ldg(a.tb.uc_stage1 + k)); }, [&](uint32_t k) { return ldg(a.tb.uc_stage2 + k); }, cp, true);
                         if (cp_is_cjk(cp)) cls |= A_CJK;
+                        if (family == 4) {
+                            // Gemma-3 shape: only a whole character, strictly well formed and inside its document, has a class
+                            const bool c1 = (b1 & 0xC0u) == 0x80u, c2 = (b2 & 0xC0u) == 0x80u, c3 = (b3 & 0xC0u) == 0x80u;
+                            bool whole = false;
+                            if (b >= 0xC2u && b <= 0xDFu) whole = avail >= 2 && c1;
+                            else if ((b & 0xF0u) == 0xE0u) whole = avail >= 3 && c1 && c2 && cp >= 0x800u && !(cp >= 0xD800u && cp <= 0xDFFFu);
+                            else if (b >= 0xF0u && b <= 0xF4u) whole = avail >= 4 && c1 && c2 && c3 && cp >= 0x10000u && cp <= 0x10FFFFu;
+                            if (!whole) cls = A_O;
+                            else if (cp == 0x2581u) cls |= A_SP;
+                        }
                     } else if (cp < 0x10000u) {
                         const uint32_t leaf = sm.ucs1[cp >> 7];
                         cls = (sm.ucs2[leaf * 8u + ((cp & 127u) >> 4)] >> ((cp & 15u) * 2u)) & 3u;
@@ -1756,13 +1717,13 @@ GTOK_DEV void pretok_tile(Blk& blk, const EncodeArgs& a, PretokSmem& sm, int til
                         cls = (ldg(a.tb.uc_stage2 + leaf * 8u + ((cp & 127u) >> 4)) >> ((cp & 15u) * 2u)) & 3u;
                     }
                     sm.attr[i0 + i] = static_cast<uint8_t>(cls | (sm.attr[i0 + i] & A_DOC));
-                    sm.oh[i0 + i] = onehot_of(static_cast<uint8_t>(cls & A_CLS));
+                    sm.oh[i0 + i] = onehot_of(static_cast<uint8_t>(cls & (A_CLS | A_SP)));
                 }
                 ow[0] = ohw[0]; ow[1] = ohw[1]; ow[2] = ohw[2]; ow[3] = ohw[3];
                 if (kWide) { aw[0] = atw[0]; aw[1] = atw[1]; aw[2] = atw[2]; aw[3] = atw[3]; }
             }
             chunk_planes(sm, c, ow, tw);
-            if (kWide) chunk_xplanes(sm, c, aw, tw);
+            if (kWide) chunk_xplanes(sm, c, aw, tw, family == 4);
             sm.cand16[c] = static_cast<uint16_t>(cand);
         }
     });
@@ -1857,7 +1818,7 @@ GTOK_DEV void pretok_tile(Blk& blk, const EncodeArgs& a, PretokSmem& sm, int til
                     if (kWide) {
                         const uint32_t* awp = reinterpret_cast<const uint32_t*>(sm.attr + c * 16);
                         const uint32_t aw[4] = {awp[0], awp[1], awp[2], awp[3]};
-                        chunk_xplanes(sm, c, aw, tw);
+                        chunk_xplanes(sm, c, aw, tw, family == 4);
                     }
                 }
             });
@@ -1874,7 +1835,7 @@ GTOK_DEV void pretok_tile(Blk& blk, const EncodeArgs& a, PretokSmem& sm, int til
         const uint32_t last_b = w.vhi - 1 >= w.vlo ? sm.txt[w.vhi - 1 - lo] : 0u, first_b = w.vlo < w.vhi ? sm.txt[w.vlo - lo] : 0u;
         const bool fwd = w.vhi < n && (last_b == 0x20u || last_b == 0x09u || last_b == 0x0Bu || last_b == 0x0Cu);
         const bool back = w.vlo >= 2 && (first_b == 0x0Au || first_b == 0x0Du);
-        if (!a.tb.added_ws && (fwd || back)) far_runs(blk, a, sm, lo, w.vlo, w.vhi, n);
+        if (!a.tb.added_ws && (fwd || back) && !(kWide && family == 4)) far_runs(blk, a, sm, lo, w.vlo, w.vhi, n);
     }
 
     // ---- P3: boundary bits, 32 bytes per thread as 64-bit planes with 16-bit margins ----
@@ -1916,19 +1877,31 @@ GTOK_DEV void pretok_tile(Blk& blk, const EncodeArgs& a, PretokSmem& sm, int til
         // (a continuation byte right after an apostrophe stretches a contraction past three bytes)
         // An added-token literal is its start bit plus continuation bits; those long stretches are
         // harmless to the algebra (the literal has no class, so its neighbours see "nothing").
+        // (planes of the wide class table)
+        auto xload = [&](int k) -> uint64_t {
+            const uint32_t* pw = reinterpret_cast<const uint32_t*>(xplane(sm, k));
+            return (static_cast<uint64_t>(pw[ww - 1]) >> 16) | (static_cast<uint64_t>(pw[ww]) << 16) | (static_cast<uint64_t>(pw[ww + 1]) << 48);
+        };
+        (void)xload;
         if (kWide && family == 4) {
-            // Gemma-3 shape: every byte outside an added-token literal is decided one by one (is_boundary_sp)
-            unc = ~(ADraw & C);
-            for (int bit = 16; bit < 48; ++bit) {
-                const int p = lo + ww * 32 + bit - 16;
-                if (p < 0 || p >= n) unc &= ~(1ull << bit);
-            }
+            // Gemma-3 shape.  The model merges the characters of the whole text, so any cut must be one that no rule can reach
+            // across.  Two kinds are taken.  A byte that is not part of a whole character of the vocabulary (a character the
+            // vocabulary lacks, malformed UTF-8, a character cut by a document's end) stands alone: the model spells it as its
+            // "<0xNN>" token, which no rule mentions, and keeping such bytes apart is also what keeps the loader's
+            // byte-to-character rules from ever seeing them.  And a space (U+0020, which the normaliser writes as U+2581, or
+            // that character itself) opens a pre-token unless some rule's left side ends with the character before it while its
+            // right side begins with U+2581 (class 6 in the vocabulary's class table; 0 any other character of the vocabulary,
+            // 3 everything else).  A character reaches at most three bytes on, so the margin settles every case.
+            // (With every byte decoded by itself, one by one, this kernel took 310 us for 300 KB.)
+            const uint64_t P6 = xload(XP_PS) & ~ADraw, K = (L & ~ADraw) | P6, W2 = xload(XP_W2), W3 = xload(XP_W3), W4 = xload(XP_W4);
+            auto cover = [&](uint64_t lead) -> uint64_t { return lead | ((lead & W2) << 1) | ((lead & W3) << 2) | ((lead & W4) << 3); };
+            const uint64_t whole = cover(K), joins = cover(P6);          // bytes of whole characters; of those a rule may join to a U+2581
+            bnd = DOC | ~whole | (K & (~(whole << 1) | (SP & ~(joins << 1))));
+            bnd = (bnd & ~(ADraw & C)) | AD;
+            const int left = n - (lo + ww * 32);
+            if (left < 32) bnd &= left <= 0 ? 0ull : ((1ull << (16 + left)) - 1ull);
         } else if (kWide) {
             // DeepSeek-V3 (see is_boundary_deepseek for the rules; here the same over whole planes).
-            auto xload = [&](int k) -> uint64_t {
-                const uint32_t* pw = reinterpret_cast<const uint32_t*>(xplane(sm, k));
-                return (static_cast<uint64_t>(pw[ww - 1]) >> 16) | (static_cast<uint64_t>(pw[ww]) << 16) | (static_cast<uint64_t>(pw[ww + 1]) << 48);
-            };
             const uint64_t PS = xload(XP_PS), AL = xload(XP_AL), APU = xload(XP_APU), CJ = xload(XP_CJK);
             const uint64_t Op = O & ~PS;                        // the O plane holds punctuation and symbols too
             const uint64_t Cg = C & ~ADraw;
@@ -2073,19 +2046,8 @@ GTOK_DEV void pretok_tile(Blk& blk, const EncodeArgs& a, PretokSmem& sm, int til
             const uint8_t a0 = sm.attr[i];
             const uint64_t m = 1ull << bit;
             if ((a0 & A_CLS) == A_ADDED) { bnd |= m; continue; }
-            if (kWide && family == 4 && i >= 1) {
-                // Gemma-3 shape, an ASCII character after an ASCII character of the same document, no added token before it: settled
-                // from two bit sets of the vocabulary's ASCII characters (is_boundary_sp says the same, by the long way)
-                const uint32_t c = sm.txt[i], c1 = sm.txt[i - 1];
-                if (c < 0x80u && c1 < 0x80u && p >= 1 && !((DOC >> bit) & 1ull) && !((ADraw >> (bit - 1)) & 1ull)) {
-                    const bool known = (a.tb.sp_ascii_known[c >> 5] >> (c & 31)) & 1u, known1 = (a.tb.sp_ascii_known[c1 >> 5] >> (c1 & 31)) & 1u;
-                    const bool cut = !known || !known1 || (c == 0x20u && !((a.tb.sp_ascii_before_bar[c1 >> 5] >> (c1 & 31)) & 1u));
-                    if (cut) bnd |= m; else bnd &= ~m;
-                    continue;
-                }
-            }
             bool pending = false, ns = false;
-            const bool bb = kWide ? (family == 4 ? is_boundary_sp(w, p) : is_boundary_deepseek(w, p, a0, &pending, &ns)) : is_boundary(w, p, a0, family, &pending, &ns);
+            const bool bb = kWide ? is_boundary_deepseek(w, p, a0, &pending, &ns) : is_boundary(w, p, a0, family, &pending, &ns);
             if (bb) bnd |= m; else bnd &= ~m;
             if (pending) pend |= m; else pend &= ~m;
             if ((a0 & A_CLS) == A_N) { if (ns) nstart |= m; else nstart &= ~m; }
