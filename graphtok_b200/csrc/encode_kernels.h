@@ -21,7 +21,6 @@ void launch_docmask(const EncodeArgs& a, uint32_t* docmask, int blocks, cudaStre
 void launch_raw_docmask(const EncodeArgs& a, uint32_t* docmask, int blocks, cudaStream_t s);   // over raw_doc_off
 // check: the context's arguments with raw_docmask unset; copy and nfc: the context's own arguments
 void launch_nfc_check(const EncodeArgs& a, int blocks, cudaStream_t s);
-void launch_nfc_copy(const EncodeArgs& a, int blocks, cudaStream_t s);
 void launch_nfc(const EncodeArgs& a, int blocks, cudaStream_t s);
 void launch_pretok(const EncodeArgs& a, int blocks, cudaStream_t s);
 void launch_words(const EncodeArgs& a, int blocks, cudaStream_t s);

@@ -621,7 +621,7 @@ struct Engine::Impl {
         }
     }
 
-    // Normalisation, in three launches: look for codepoints that can make the raw text non-NFC; if
+    // Normalisation, in two launches: look for codepoints that can make the raw text non-NFC; if
     // there are none (the usual case) copy text and header over as they are; else normalise.  The
     // second and third each return at once in the case that is not theirs.
     void launch_normalise(Ctx* c) {
@@ -629,7 +629,6 @@ struct Engine::Impl {
         chk.raw_docmask = nullptr;
         const int wide = std::max(1, std::min<int>(static_cast<int>(c->n_tiles_cap) * 2, sm_count * 8));
         launch_nfc_check(chk, wide, c->stream);
-        launch_nfc_copy(c->args, wide, c->stream);
         if (c->batch) {
             cudaMemsetAsync(c->d_docmask_raw, 0, c->mask_words * 4, c->stream);
             launch_raw_docmask(c->args, c->d_docmask_raw, c->docmask_blocks, c->stream);
