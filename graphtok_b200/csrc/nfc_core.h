@@ -27,10 +27,12 @@ namespace gtok {
 constexpr int kNfcMaxCps = 96;       // decomposed codepoints of one stretch; longer ones are flagged (kErrNfcLong)
 
 constexpr int kNfcStage = kTile + 528;      // bytes of a tile's output put together in shared memory before they go out
+constexpr uint32_t kNfcKeep = 28;           // bytes of normalised stretches a chunk keeps (the sixteen bytes of a chunk rarely own more)
 struct NfcSmem {
     alignas(16) uint8_t outb[kNfcStage];
-    uint8_t sres[kThreads][12];      // the normalised form of the one stretch a chunk owns, kept from sizing to writing
-    uint8_t slen[kThreads];          // its length; 0: not kept (no stretch, several, or longer than that)
+    uint8_t sres[kThreads][kNfcKeep];     // the normalised forms of the first stretches a chunk owns, one after the other, kept from sizing to writing
+    uint32_t slen[kThreads];         // their lengths, four bits each, the first in the lowest
+    uint8_t scnt[kThreads];          // how many are kept
     uint32_t scan[kThreads];
     uint16_t attl[kThreads + 2];     // per 16-byte chunk, one before and one after the tile: attention lead bytes
     uint16_t attf[kThreads + 2];     // ... and every byte of an attention codepoint
@@ -343,7 +345,8 @@ GTOK_DEV void nfc_tile(Blk& blk, const EncodeArgs& a, NfcSmem& sm, int tile) {
                                       (static_cast<unsigned long long>(sm.attl[tid + 2]) << 32);
         const unsigned long long wf = static_cast<unsigned long long>(sm.attf[tid]) | (static_cast<unsigned long long>(sm.attf[tid + 1]) << 16) |
                                       (static_cast<unsigned long long>(sm.attf[tid + 2]) << 32);
-        uint32_t drop = sm.attf[tid + 1], own = 0, extra = 0, kept = 0;
+        uint32_t drop = sm.attf[tid + 1], own = 0, extra = 0, kept = 0, n_kept = 0, lens = 0;
+        bool keep = true;
         // run starts at c0 .. c0 + 19: the codepoint before such a run may lie in this chunk
         unsigned long long rs = wl & ~(wf << 1);
         if (a.raw_docmask && (wl >> 16)) {
@@ -371,15 +374,17 @@ GTOK_DEV void nfc_tile(Blk& blk, const EncodeArgs& a, NfcSmem& sm, int tile) {
             if (a0 >= c0 && a0 < c0 + kPer) {
                 own |= 1u << (a0 - c0);
                 drop |= 1u << (a0 - c0);
-                // (the first one's bytes are kept for the write phase when they fit: working a stretch out is one thread's
-                // job while its warp waits, and most of what this kernel costs)
-                const bool keep = own == (1u << (a0 - c0));
-                const uint32_t len = nfc_stretch(a, a0, p, n, keep ? sm.sres[tid] : nullptr, 0, keep ? 12u : 0u);
-                kept = keep && len <= 12u ? len : 0u;
+                // (the bytes are kept for the write phase as far as they fit: working a stretch out is one thread's job while
+                // its warp waits, and most of what this kernel costs; with only the one stretch of a chunk kept, chunks of two
+                // and more, usual where a word has several marks, were worked out twice)
+                const uint32_t len = nfc_stretch(a, a0, p, n, keep ? sm.sres[tid] : nullptr, kept, keep ? kNfcKeep : 0u);
+                if (keep && len < 16u && kept + len <= kNfcKeep && n_kept < 8u) { lens |= len << (4 * n_kept); kept += len; ++n_kept; }
+                else keep = false;
                 extra += len;
             }
         }
-        sm.slen[tid] = static_cast<uint8_t>(popc32(own) == 1 ? kept : 0u);
+        sm.slen[tid] = lens;
+        sm.scnt[tid] = static_cast<uint8_t>(n_kept);
         sm.drop[tid] = static_cast<uint16_t>(drop);
         sm.own[tid] = static_cast<uint16_t>(own);
         sm.scan[tid] = static_cast<uint32_t>(popc32(valid & ~drop)) + extra;
@@ -415,6 +420,8 @@ GTOK_DEV void nfc_tile(Blk& blk, const EncodeArgs& a, NfcSmem& sm, int tile) {
                 else for (int i = 0; i < kPer; ++i) sm.outb[la + i] = static_cast<uint8_t>(w[i >> 2] >> (8 * (i & 3)));
                 return;
             }
+            const uint32_t n_kept = sm.scnt[tid];
+            uint32_t kept = 0, k = 0, lens = sm.slen[tid];
             for (uint32_t i = 0; i < cnt; ++i) {
                 if ((docbits >> i) & 1u) {
                     const uint32_t r = c0 + i;
@@ -423,15 +430,19 @@ GTOK_DEV void nfc_tile(Blk& blk, const EncodeArgs& a, NfcSmem& sm, int tile) {
                     for (uint32_t d = lo; d <= n_docs && ldg(a.raw_doc_off + d) == r; ++d) a.norm_doc_off[d] = base + (la - shift);
                 }
                 if ((own >> i) & 1u) {
+                    if (k++ < n_kept) {
+                        const uint32_t len = lens & 15u;
+                        for (uint32_t t = 0; t < len; ++t) sm.outb[la + t] = sm.sres[tid][kept + t];
+                        lens >>= 4; kept += len; la += len;
+                        continue;
+                    }
                     const uint32_t a0 = c0 + i;
                     uint32_t p = a0;
                     if (!((sm.attl[tid + 1] >> i) & 1u)) {
                         uint32_t cp;
                         p = a0 + static_cast<uint32_t>(nfc_decode(a, a0, n, &cp));
                     }
-                    const uint32_t kept = sm.slen[tid];
-                    if (kept) { for (uint32_t t = 0; t < kept; ++t) sm.outb[la + t] = sm.sres[tid][t]; la += kept; }
-                    else la += nfc_stretch(a, a0, p, n, sm.outb, la, kNfcStage);
+                    la += nfc_stretch(a, a0, p, n, sm.outb, la, kNfcStage);
                 } else if (!((drop >> i) & 1u)) {
                     sm.outb[la] = static_cast<uint8_t>(w[i >> 2] >> (8 * (i & 3)));
                     ++la;
