@@ -2761,43 +2761,71 @@ GTOK_DEV void put_id(const EncodeArgs& a, uint32_t g, uint32_t k, uint32_t id) {
 // The first two phases of a batch over the block's arena (sm.word holds the batch's entries, position |
 // length << 32, 0 = none): all threads fetch the bytes, a slot each, so that the loads overlap ...
 constexpr uint32_t kPendingRank = 0xFFFFFFFDu;
+// Where slot x of the arena belongs, for x = tid, tid + kThreads, ...: pre-token w, group of four slots g.  (Stepped along, not
+// divided out at every slot.  With that and two look-ups in flight a thread in place of one: merge kernel on a 32 MB corpus file
+// 439 -> 421 us, 27 MB of documents 134 -> 128, 8.5 MB of code 163 -> 157, a 4.5 MB document 69 -> 67.)
+struct ArenaWalk {
+    uint32_t w, g, batch, dw, dg;
+    GTOK_DEV ArenaWalk(uint32_t tid, uint32_t n_batch) : w((tid >> 2) % n_batch), g((tid >> 2) / n_batch), batch(n_batch), dw((kThreads / 4) % n_batch), dg((kThreads / 4) / n_batch) {}
+    GTOK_DEV void step() { w += dw; g += dg; if (w >= batch) { w -= batch; ++g; } }
+};
 template <class Blk>
 GTOK_DEV void arena_fill(Blk& blk, const EncodeArgs& a, MissSmem& sm, uint32_t* ids, uint32_t* rk, uint32_t batch, uint32_t max_len) {
     const uint32_t slots = batch * max_len;
     blk.par([&](int tid) {
-        for (uint32_t x = tid; x < slots; x += kThreads) {
-            const uint32_t w = (x >> 2) % batch, r = ((x >> 2) / batch) * 4u + (x & 3u);
-            const unsigned long long wv = sm.word[w];
-            const uint32_t g = static_cast<uint32_t>(wv), len = static_cast<uint32_t>(wv >> 32);
-            if (r >= ((len + 3u) & ~3u)) continue;                  // beyond the pre-token's last group: never read
-            if (r >= len) { rk[x] = kNoRank; continue; }            // padding of the last group
-            const uint32_t bt = ldg(a.text + g + r);
-            sm.rawb[w * max_len + r] = static_cast<uint8_t>(bt);
-            ids[x] = sm.b2i[bt];
-            rk[x] = (r + 1 < len) ? kPendingRank : kNoRank;
-            sm.lnk[x] = static_cast<uint16_t>(((r ? r - 1 : 0xFFu) << 8) | (r + 1 < len ? r + 1 : 0xFFu));
+        ArenaWalk at(tid, batch);
+        for (uint32_t x0 = tid; x0 < slots; x0 += 2 * kThreads) {
+            // two slots at a time, so that their bytes are requested together
+            uint32_t bt[2], r[2], len[2], w[2];
+            GTOK_UNROLL
+            for (int u = 0; u < 2; ++u) {
+                w[u] = at.w; r[u] = at.g * 4u + (tid & 3u); bt[u] = 0; len[u] = 0;
+                at.step();
+                if (x0 + u * kThreads >= slots) continue;
+                const unsigned long long wv = sm.word[w[u]];
+                len[u] = static_cast<uint32_t>(wv >> 32);
+                if (r[u] < len[u]) bt[u] = ldg(a.text + static_cast<uint32_t>(wv) + r[u]);
+            }
+            GTOK_UNROLL
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t x = x0 + u * kThreads;
+                if (x >= slots || r[u] >= ((len[u] + 3u) & ~3u)) continue;      // beyond the pre-token's last group: never read
+                if (r[u] >= len[u]) { rk[x] = kNoRank; continue; }              // padding of the last group
+                sm.rawb[w[u] * max_len + r[u]] = static_cast<uint8_t>(bt[u]);
+                ids[x] = sm.b2i[bt[u]];
+                rk[x] = (r[u] + 1 < len[u]) ? kPendingRank : kNoRank;
+                sm.lnk[x] = static_cast<uint16_t>(((r[u] ? r[u] - 1 : 0xFFu) << 8) | (r[u] + 1 < len[u] ? r[u] + 1 : 0xFFu));
+            }
         }
     });
 }
-// ... and probe all adjacent pairs, a slot each; then the lowest key of every group of four slots
+// ... and probe all adjacent pairs, a slot each, two in flight a thread; then the lowest key of every group of four slots
 // (pre-tokens of more than 16 bytes search through these).
 template <class Blk>
 GTOK_DEV void arena_pairs(Blk& blk, const EncodeArgs& a, MissSmem& sm, uint32_t* ids, uint32_t* rk, uint32_t* nw, uint32_t batch, uint32_t max_len) {
     const uint32_t slots = batch * max_len, stride = batch * 4u;
     blk.par([&](int tid) {
-        for (uint32_t x = tid; x < slots; x += kThreads) {
-            const uint32_t w = (x >> 2) % batch, r = ((x >> 2) / batch) * 4u + (x & 3u);
-            const uint32_t len = static_cast<uint32_t>(sm.word[w] >> 32);
-            if (r + 1 >= len || rk[x] != kPendingRank) continue;
-            RankRes q = probe_rule(a.tb, ids[x], ids[arena_at(4u * w, stride, r + 1)]);
-            rk[x] = rank_key(q.rank, r);
-            nw[x] = q.res;
+        ArenaWalk at(tid, batch);
+        for (uint32_t x0 = tid; x0 < slots; x0 += 2 * kThreads) {
+            const uint32_t x1 = x0 + kThreads, w0 = at.w, r0 = at.g * 4u + (tid & 3u);
+            at.step();
+            const uint32_t w1 = at.w, r1 = at.g * 4u + (tid & 3u);
+            at.step();
+            const bool do0 = r0 + 1 < static_cast<uint32_t>(sm.word[w0] >> 32) && rk[x0] == kPendingRank;
+            const bool do1 = x1 < slots && r1 + 1 < static_cast<uint32_t>(sm.word[w1] >> 32) && rk[x1] == kPendingRank;
+            RankRes q0, q1;
+            probe_rule2(a.tb, do0, do0 ? ids[x0] : 0u, do0 ? ids[arena_at(4u * w0, stride, r0 + 1)] : 0u, &q0,
+                        do1, do1 ? ids[x1] : 0u, do1 ? ids[arena_at(4u * w1, stride, r1 + 1)] : 0u, &q1);
+            if (do0) { rk[x0] = rank_key(q0.rank, r0); nw[x0] = q0.res; }
+            if (do1) { rk[x1] = rank_key(q1.rank, r1); nw[x1] = q1.res; }
         }
     });
     if (max_len > 16u) {
         blk.par([&](int tid) {
+            ArenaWalk at(tid, batch);
             for (uint32_t i = tid; i < slots / 4u; i += kThreads) {
-                const uint32_t w = (i >> 2) % batch, g = ((i >> 2) / batch) * 4u + (i & 3u);
+                const uint32_t w = at.w, g = at.g * 4u + (tid & 3u);
+                at.step();
                 const uint32_t len = static_cast<uint32_t>(sm.word[w] >> 32);
                 uint32_t m = kNoRank;
                 if (g * 4u < len) for (uint32_t r = g * 4u; r < g * 4u + 4u; ++r) { const uint32_t v = rk[arena_at(4u * w, stride, r)]; if (v < m) m = v; }
