@@ -2,9 +2,10 @@
 
 The product is `lib/libgtok.so` (CUDA kernels + C++ engine + extern "C" boundary,
 built by `python -m graphtok_b200.build`).  This package only locates and binds it
-through ctypes (the calls that take or return Python text, lists and arrays through the extension
-`_host`, which the same build makes); it has no CPU implementation of the encode path, and
-`GTok(...)` raises when the library or a B200 is missing.
+through ctypes.  The calls that take or return Python text, lists and arrays go through the extension
+`_host`, which the same build makes where Python's and numpy's headers are there, and else through
+`ctypes_host`.  The package has no CPU implementation of the encode path, and `GTok(...)` raises when
+the library or a B200 is missing.
 """
 import ctypes
 import os
@@ -97,8 +98,12 @@ def load_lib():
     lib.gtok_x_plan_documents.argtypes = [vp, u32, u32, vp]
     lib.gtok_x_table_bytes.restype = None
     lib.gtok_x_table_bytes.argtypes = [vp, vp]
-    from . import _host                      # built beside the library; it binds to the same libgtok.so
-    lib.host = _host
+    try:
+        from . import _host as host          # built beside the library where the interpreter's headers are
+    except ImportError:
+        from .ctypes_host import CtypesHost
+        host = CtypesHost(lib)
+    lib.host = host
     lib.gtok_x_launches_per_replay.restype = i32
     lib.gtok_x_launches_per_replay.argtypes = [vp, i32]
     _lib = lib

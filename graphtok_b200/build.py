@@ -3,7 +3,8 @@
   graphtok_b200/lib/libgtok.so      CUDA kernels + engine + C ABI, sm_100a only
   graphtok_b200/datagen/datagen     synthetic text / vocabulary generator (host only)
   graphtok_b200/cli/gpu_bpe_tokenize   command-line tool over libgtok.so
-  graphtok_b200/_host.so            CPython extension: Python objects to and from libgtok.so
+  graphtok_b200/_host.so            CPython extension: Python objects to and from libgtok.so (left out,
+                                    with a line that says so, where Python's or numpy's headers are missing)
 
 nvcc cross-compiles without a GPU.  Run as `python -m graphtok_b200.build`.
 """
@@ -84,17 +85,39 @@ def build_cli(force=False):
 HOST = os.path.join(HERE, "_host.so")
 
 
-def build_host(force=False):
-    """The CPython extension between the Python classes and libgtok.so."""
+def _host_includes():
+    """Folders with the headers of this interpreter and of numpy, or the name of what is missing."""
     import sysconfig
+    python = [d for d in (sysconfig.get_paths().get(k) for k in ("include", "platinclude")) if d and os.path.exists(os.path.join(d, "Python.h"))]
+    if not python:
+        return "Python.h"
+    try:
+        import numpy
+    except ImportError:
+        return "numpy"
+    if not os.path.exists(os.path.join(numpy.get_include(), "numpy", "arrayobject.h")):
+        return "numpy/arrayobject.h"
+    return python[:1] + [numpy.get_include()]
 
-    import numpy
+
+def build_host(force=False):
+    """The CPython extension between the Python classes and libgtok.so; None where it cannot be built, and the classes
+    then go by ctypes (ctypes_host.py)."""
     src = os.path.join(HERE, "pyhost", "host_module.cc")
     if not force and not _newer(HOST, [src, os.path.join(HERE, "..", "include", "gtok.h"), LIB]):
         return HOST
-    subprocess.run(["g++", "-std=c++17", "-O3", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"], "-I" + numpy.get_include(),
-                    "-o", HOST, src, "-L" + LIB_DIR, "-l:libgtok.so", "-Wl,-rpath,$ORIGIN/lib"], check=True)
-    return HOST
+    if os.path.exists(HOST):
+        os.remove(HOST)          # an outdated one must not be loaded
+    why = _host_includes()
+    if not isinstance(why, str):
+        cmd = ["g++", "-std=c++17", "-O3", "-fPIC", "-shared", "-fvisibility=hidden"] + ["-I" + d for d in why] + [
+            "-o", HOST, src, "-L" + LIB_DIR, "-l:libgtok.so", "-Wl,-rpath,$ORIGIN/lib"]
+        done = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if done.returncode == 0:
+            return HOST
+        why = next((line for line in done.stdout.splitlines() if "error" in line), "g++ exit code %d" % done.returncode)
+    print("graphtok_b200: extension _host left out, ctypes in its place (%s)" % why, flush=True)
+    return None
 
 
 def main():
@@ -102,11 +125,12 @@ def main():
     build_lib(force=force, verbose="-v" in sys.argv)
     build_datagen(force=force)
     build_cli(force=force)
-    build_host(force=force)
+    host = build_host(force=force)
     print(LIB)
     print(DATAGEN)
     print(CLI)
-    print(HOST)
+    if host:
+        print(host)
 
 
 if __name__ == "__main__":

@@ -16,20 +16,13 @@ import os
 import numpy as np
 
 from .. import GTok, GTokError, load_lib
+from ..ctypes_host import as_bytes as _as_bytes
 
 __all__ = ["Tokenizer", "Dispatcher"]
 
 _KINDS = {0: "GPT2", 1: "Llama3", 2: "Qwen25", 3: "DeepSeekV3", 4: "Gemma3"}
 _POLICIES = {"adaptive": 0, "gpu": 1, "cpu": 2}
 _BACKENDS = ("", "auto", "off", "host", "gigatoken")
-
-
-def _as_bytes(text):
-    if isinstance(text, str):
-        return text.encode("utf-8")
-    if isinstance(text, (bytes, bytearray, memoryview)):
-        return bytes(text)
-    raise TypeError("text must be str or bytes")
 
 
 def _device_words(n):

@@ -66,10 +66,17 @@ def test_utf8_form(utf8, width, kind, n):
             assert utf8.size(units.ctypes.data, n, kind) == 0xFFFFFFFFFFFFFFFF
 
 
-@pytest.fixture(scope="module")
-def tok():
+@pytest.fixture(scope="module", params=["extension", "ctypes"])
+def tok(request):
+    """A tokenizer that goes by the extension, and one that goes by ctypes as where the extension was not built."""
+    from graphtok_b200.ctypes_host import CtypesHost
     from graphtok_b200.gpu_bpe_tokenizer import Tokenizer
-    return Tokenizer(tiny_vocab("llama3"))
+    t = Tokenizer(tiny_vocab("llama3"))
+    if request.param == "ctypes":
+        t._host = t._g.host = CtypesHost(t._g.lib)
+    elif isinstance(t._host, CtypesHost):
+        pytest.skip("the extension is not built here")
+    return t
 
 
 # sizes: single-block route and its limit, one copy step and several, the size from which characters are shared among
