@@ -100,6 +100,7 @@ def load_lib():
     lib.gtok_x_table_bytes.argtypes = [vp, vp]
     try:
         from . import _host as host          # built beside the library where the interpreter's headers are
+        host.bind(lambda name: ctypes.cast(getattr(lib, name), vp).value)
     except ImportError:
         from .ctypes_host import CtypesHost
         host = CtypesHost(lib)

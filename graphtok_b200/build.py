@@ -104,14 +104,14 @@ def build_host(force=False):
     """The CPython extension between the Python classes and libgtok.so; None where it cannot be built, and the classes
     then go by ctypes (ctypes_host.py)."""
     src = os.path.join(HERE, "pyhost", "host_module.cc")
-    if not force and not _newer(HOST, [src, os.path.join(HERE, "..", "include", "gtok.h"), LIB]):
+    if not force and not _newer(HOST, [src, os.path.join(HERE, "..", "include", "gtok.h")]):
         return HOST
     if os.path.exists(HOST):
         os.remove(HOST)          # an outdated one must not be loaded
     why = _host_includes()
     if not isinstance(why, str):
         cmd = ["g++", "-std=c++17", "-O3", "-fPIC", "-shared", "-fvisibility=hidden"] + ["-I" + d for d in why] + [
-            "-o", HOST, src, "-L" + LIB_DIR, "-l:libgtok.so", "-Wl,-rpath,$ORIGIN/lib"]
+            "-o", HOST, src]
         done = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if done.returncode == 0:
             return HOST

@@ -5,6 +5,8 @@
 // list one by one) and writes ids and bytes to the object that is returned, so a call makes no intermediate
 // Python object and no copy that the transfer to or from the GPU does not need.  Every function takes the
 // handle as an integer and answers an error of the library with its (negative) code as an int.
+// The module is not linked against the library: bind() takes the calls' addresses from whoever has loaded it, so
+// that there is one copy of it in the process whatever else goes by the name libgtok.so on the library path.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #define NPY_NO_DEPRECATED_API NPY_1_7_API_VERSION
@@ -23,7 +25,43 @@ namespace {
 // buffer takes less than a transfer of its own would).
 constexpr uint64_t kBlockBytes = 256 << 10;
 
-void* handle_of(PyObject* o) { return PyLong_CheckExact(o) ? PyLong_AsVoidPtr(o) : nullptr; }
+// The library's calls by address.
+struct Lib {
+    decltype(&gtok_x_set_max_bytes) set_max_bytes;
+    decltype(&gtok_x_measure) measure;
+    decltype(&gtok_x_encode_measured) encode_measured;
+    decltype(&gtok_x_take_ids) take_ids;
+    decltype(&gtok_x_decode_room) decode_room;
+    decltype(&gtok_x_decode_run) decode_run;
+    decltype(&gtok_x_take_bytes) take_bytes;
+    decltype(&gtok_x_block_get) block_get;
+    decltype(&gtok_x_block_put) block_put;
+} lib;
+bool bound = false;
+struct Need { const char* name; void* at; };
+#define GTOK_NEED(f) {"gtok_x_" #f, &lib.f}
+const Need kNeeds[] = {GTOK_NEED(set_max_bytes), GTOK_NEED(measure), GTOK_NEED(encode_measured), GTOK_NEED(take_ids), GTOK_NEED(decode_room),
+                       GTOK_NEED(decode_run), GTOK_NEED(take_bytes), GTOK_NEED(block_get), GTOK_NEED(block_put)};
+
+// bind(address): address(name) -> where that call of gtok.h is in the loaded library.
+PyObject* py_bind(PyObject*, PyObject* address) {
+    for (const Need& n : kNeeds) {
+        PyObject* at = PyObject_CallFunction(address, "s", n.name);
+        void* p = at ? PyLong_AsVoidPtr(at) : nullptr;
+        Py_XDECREF(at);
+        if (!p) {
+            if (!PyErr_Occurred()) PyErr_Format(PyExc_ImportError, "no %s in the library", n.name);
+            bound = false;
+            return nullptr;
+        }
+        std::memcpy(n.at, &p, sizeof p);
+    }
+    bound = true;
+    Py_RETURN_NONE;
+}
+
+// A handle of the bound library; none before there is one.
+void* handle_of(PyObject* o) { return bound && PyLong_CheckExact(o) ? PyLong_AsVoidPtr(o) : nullptr; }
 
 // The texts of one call: where each lies, and what keeps it there until the call is over.
 struct Texts {
@@ -77,23 +115,23 @@ struct Texts {
 
 // The byte cap doubled until a text of `bytes` fits even if normalisation lengthens it (at most threefold).
 void grow_cap(void* h, int64_t bytes) {
-    uint64_t cap = gtok_x_set_max_bytes(h, 0);
+    uint64_t cap = lib.set_max_bytes(h, 0);
     const uint64_t need = static_cast<uint64_t>(bytes) * 3 + 64;
     if (!cap || cap >= need) return;
     while (cap < need) cap *= 2;
-    gtok_x_set_max_bytes(h, static_cast<uint32_t>(std::min<uint64_t>(cap, 0xFFFFFFFFull)));
+    lib.set_max_bytes(h, static_cast<uint32_t>(std::min<uint64_t>(cap, 0xFFFFFFFFull)));
 }
 
-void release_block(PyObject* capsule) { gtok_x_block_put(PyCapsule_GetPointer(capsule, nullptr)); }
+void release_block(PyObject* capsule) { lib.block_put(PyCapsule_GetPointer(capsule, nullptr)); }
 
 // An array for `n` ids.
 PyObject* new_ids(int64_t n) {
     npy_intp dim = static_cast<npy_intp>(n);
     if (static_cast<uint64_t>(n) * 4 >= kBlockBytes) {
-        if (void* p = gtok_x_block_get(static_cast<uint64_t>(n) * 4)) {
+        if (void* p = lib.block_get(static_cast<uint64_t>(n) * 4)) {
             PyObject* a = PyArray_SimpleNewFromData(1, &dim, NPY_UINT32, p);
             PyObject* c = a ? PyCapsule_New(p, nullptr, release_block) : nullptr;
-            if (!c) { Py_XDECREF(a); gtok_x_block_put(p); return nullptr; }
+            if (!c) { Py_XDECREF(a); lib.block_put(p); return nullptr; }
             if (PyArray_SetBaseObject(reinterpret_cast<PyArrayObject*>(a), c) < 0) { Py_DECREF(a); return nullptr; }     // (the capsule is gone either way)
             return a;
         }
@@ -119,11 +157,11 @@ struct Outcome { int64_t bytes, ids; };
 Outcome encode_texts(void* h, const gtok_x_piece* p, uint32_t n, bool batch, bool grow) {
     Outcome o;
     Py_BEGIN_ALLOW_THREADS
-    o.bytes = gtok_x_measure(h, p, n, batch ? 1 : 0);
+    o.bytes = lib.measure(h, p, n, batch ? 1 : 0);
     if (o.bytes < 0) o.ids = kSurrogate;
     else {
         if (grow) grow_cap(h, o.bytes);
-        o.ids = gtok_x_encode_measured(h, o.bytes, nullptr, 0, nullptr);
+        o.ids = lib.encode_measured(h, o.bytes, nullptr, 0, nullptr);
     }
     Py_END_ALLOW_THREADS
     return o;
@@ -143,10 +181,10 @@ PyObject* py_encode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!ids) return nullptr;
     int r;
     if (static_cast<uint64_t>(o.ids) * 4 < kBlockBytes) {
-        r = gtok_x_take_ids(h, data_of(ids), nullptr);
+        r = lib.take_ids(h, data_of(ids), nullptr);
     } else {
         Py_BEGIN_ALLOW_THREADS
-        r = gtok_x_take_ids(h, data_of(ids), nullptr);
+        r = lib.take_ids(h, data_of(ids), nullptr);
         Py_END_ALLOW_THREADS
     }
     if (r < 0) { Py_DECREF(ids); return PyLong_FromLong(r); }
@@ -180,7 +218,7 @@ PyObject* py_encode_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!off) { Py_DECREF(ids); return nullptr; }
     int r;
     Py_BEGIN_ALLOW_THREADS
-    r = gtok_x_take_ids(h, data_of(ids), data_of(off));
+    r = lib.take_ids(h, data_of(ids), data_of(off));
     Py_END_ALLOW_THREADS
     if (r < 0) { Py_DECREF(ids); Py_DECREF(off); return PyLong_FromLong(r); }
     return Py_BuildValue("(NN)", ids, off);
@@ -199,7 +237,7 @@ PyObject* py_encode_to_device(PyObject*, PyObject* const* args, Py_ssize_t nargs
     const uint32_t n = batch ? static_cast<uint32_t>(t.pieces.size()) : 1u;
     int64_t bytes;
     Py_BEGIN_ALLOW_THREADS
-    bytes = gtok_x_measure(h, p, n, batch ? 1 : 0);
+    bytes = lib.measure(h, p, n, batch ? 1 : 0);
     if (bytes >= 0 && args[2] == Py_True) grow_cap(h, bytes);
     Py_END_ALLOW_THREADS
     if (bytes < 0) return batch ? raise_encode_error(PySequence_Fast_ITEMS(args[1]), PyTuple_GET_SIZE(args[1])) : raise_encode_error(args + 1, 1);
@@ -223,7 +261,7 @@ PyObject* py_encode_to_device(PyObject*, PyObject* const* args, Py_ssize_t nargs
         if (!ids) { Py_XDECREF(off); return nullptr; }
         int64_t got;
         Py_BEGIN_ALLOW_THREADS
-        got = gtok_x_encode_measured(h, bytes, ids_at, room, off_at);
+        got = lib.encode_measured(h, bytes, ids_at, room, off_at);
         Py_END_ALLOW_THREADS
         if (got == -2 && attempt == 0) { Py_DECREF(ids); continue; }
         if (got < 0) { Py_DECREF(ids); Py_XDECREF(off); return PyLong_FromLongLong(got); }
@@ -258,7 +296,7 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         n = static_cast<uint32_t>(len);
         for (Py_ssize_t i = 0; i < len; ++i)
             if (!PyLong_CheckExact(PyList_GET_ITEM(o, i))) Py_RETURN_NONE;
-        uint32_t* room = gtok_x_decode_room(h, n);
+        uint32_t* room = lib.decode_room(h, n);
         if (!room) return PyLong_FromLong(-1);
         for (Py_ssize_t i = 0; i < len; ++i) {
             int over = 0;
@@ -278,7 +316,7 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         n = static_cast<uint32_t>(len);
         if (d->kind == 'u' && width == 4) ids = static_cast<const uint32_t*>(PyArray_DATA(a));
         else {
-            uint32_t* room = gtok_x_decode_room(h, n);
+            uint32_t* room = lib.decode_room(h, n);
             if (!room) return PyLong_FromLong(-1);
             const void* s = PyArray_DATA(a);
             Py_BEGIN_ALLOW_THREADS
@@ -292,20 +330,21 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!fits) { PyErr_SetString(PyExc_ValueError, "token ids must fit 32 unsigned bits"); return nullptr; }
     int64_t total;
     Py_BEGIN_ALLOW_THREADS
-    total = gtok_x_decode_run(h, ids, n);
+    total = lib.decode_run(h, ids, n);
     Py_END_ALLOW_THREADS
     if (total < 0) return PyLong_FromLongLong(total);
     PyObject* bytes = PyBytes_FromStringAndSize(nullptr, static_cast<Py_ssize_t>(total));
     if (!bytes || total == 0) return bytes;
     int r;
     Py_BEGIN_ALLOW_THREADS
-    r = gtok_x_take_bytes(h, reinterpret_cast<uint8_t*>(PyBytes_AS_STRING(bytes)));
+    r = lib.take_bytes(h, reinterpret_cast<uint8_t*>(PyBytes_AS_STRING(bytes)));
     Py_END_ALLOW_THREADS
     if (r < 0) { Py_DECREF(bytes); return PyLong_FromLong(r); }
     return bytes;
 }
 
 PyMethodDef kMethods[] = {
+    {"bind", py_bind, METH_O, "bind(address): address(name) -> address of that call of gtok.h in the loaded library"},
     {"encode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode)), METH_FASTCALL, "encode(handle, text, grow) -> uint32 array, or an error code"},
     {"encode_batch", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode_batch)), METH_FASTCALL,
      "encode_batch(handle, texts, grow) -> (uint32 ids, uint32 offsets), or an error code"},

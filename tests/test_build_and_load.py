@@ -45,3 +45,15 @@ def test_package_without_the_extension(built):
                 "print(g.plan_documents(np.array([0, 10, 20, 30, 40]), 2).tolist(), type(g.load_lib().host).__name__)\n"
                 "from graphtok_b200.gpu_bpe_tokenizer import Tokenizer, Dispatcher\n")
     assert out.strip() == "[0, 2, 4] CtypesHost"
+
+
+def test_one_copy_of_the_library_whatever_the_library_path(built, tmp_path):
+    """Another libgtok.so first on the library path: neither loaded nor asked for its calls."""
+    from graphtok_b200 import build, load_lib
+    (tmp_path / "other.cc").write_text('extern "C" int gtok_create() { return 7; }\n')
+    subprocess.run(["g++", "-fPIC", "-shared", "-o", str(tmp_path / "libgtok.so"), str(tmp_path / "other.cc")], check=True)
+    out = child("import graphtok_b200 as g\n"
+                "kind = type(g.load_lib().host).__name__\n"
+                "paths = {line.split()[-1] for line in open('/proc/self/maps') if 'libgtok.so' in line}\n"
+                "print(kind, *paths)\n", LD_LIBRARY_PATH="%s:%s" % (tmp_path, os.environ.get("LD_LIBRARY_PATH", "")))
+    assert out.split() == [type(load_lib().host).__name__, build.LIB]
