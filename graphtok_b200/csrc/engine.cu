@@ -298,6 +298,7 @@ struct Engine::Impl {
         single.reset();
         batch.reset();
         dec.reset();
+        if (order_ev) cudaEventDestroy(order_ev);
         for (void* p : owned) cudaFree(p);
     }
 
@@ -911,6 +912,44 @@ struct Engine::Impl {
         return true;
     }
 
+    // Memory that the caller gives for results on the device may still be in use by work queued on a stream of the caller's
+    // (an allocator that works in stream order hands a block out again while its last readers wait in the queue).  The event
+    // stands behind that work; the next result copy waits for it, the encoding itself does not.
+    cudaEvent_t order_ev = nullptr;
+    int order_dev = -1;
+    bool ordered = false;
+    bool order_after(cudaStream_t stream, std::string& err) {
+        ordered = false;
+        // (a stream under capture has no work to wait for, and an event on it would draw this engine's stream into the capture)
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) { cudaGetLastError(); return true; }
+        if (capture != cudaStreamCaptureStatusNone) return true;
+        int dev = 0;
+        GTOK_CUDA(cudaGetDevice(&dev));
+        if (order_ev && order_dev != dev) { cudaEventDestroy(order_ev); order_ev = nullptr; }
+        if (!order_ev) { GTOK_CUDA(cudaEventCreateWithFlags(&order_ev, cudaEventDisableTiming)); order_dev = dev; }
+        GTOK_CUDA(cudaEventRecord(order_ev, stream));
+        ordered = true;
+        return true;
+    }
+    // ids (and a batch's offsets) to device memory of the caller's.
+    bool copy_to_device(Ctx* c, uint32_t* out, size_t words, uint32_t* out_doc_tok, size_t doc_words, std::string& err) {
+        if (ordered) GTOK_CUDA(cudaStreamWaitEvent(c->stream, order_ev, 0));
+        ordered = false;
+        if (words) GTOK_CUDA(cudaMemcpyAsync(out, c->d_out, words * 4, cudaMemcpyDeviceToDevice, c->stream));
+        if (doc_words) GTOK_CUDA(cudaMemcpyAsync(out_doc_tok, c->d_doc_tok, doc_words * 4, cudaMemcpyDeviceToDevice, c->stream));
+        GTOK_CUDA(cudaStreamSynchronize(c->stream));
+        return true;
+    }
+    // The offsets of a batch without text.
+    bool clear_on_device(uint32_t* out_doc_tok, size_t doc_words, std::string& err) {
+        if (ordered) GTOK_CUDA(cudaEventSynchronize(order_ev));
+        ordered = false;
+        GTOK_CUDA(cudaMemset(out_doc_tok, 0, doc_words * 4));
+        GTOK_CUDA(cudaStreamSynchronize(nullptr));
+        return true;
+    }
+
     static constexpr int64_t kNoCtx = INT64_MIN;
 
     // Stages the input and replays the graph.  With NFC two things can make the first replay
@@ -1078,9 +1117,7 @@ int64_t Engine::encode(const uint8_t* text, uint32_t len, uint32_t cap_bytes, ui
     if (static_cast<uint64_t>(total) > max_out) { last_error_ = "more token ids than the output buffer holds"; return -2; }
     if (total == 0) return 0;
     if (out_on_device) {
-        cudaError_t e = cudaMemcpyAsync(out, c->d_out, static_cast<size_t>(total) * 4, cudaMemcpyDeviceToDevice, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) { last_error_ = std::string("token copy: ") + cudaGetErrorString(e); return -1; }
+        if (!im.copy_to_device(c, out, static_cast<size_t>(total), nullptr, 0, last_error_)) return -1;
     } else if (!im.copy_out(c, out, static_cast<size_t>(total), nullptr, 0, last_error_)) return -1;
     return total;
 }
@@ -1091,7 +1128,7 @@ int64_t Engine::encode_batch(const uint8_t* bytes, const uint32_t* doc_off, uint
     cudaSetDevice(im.device);
     const uint32_t len = doc_off[n_docs];
     if (len == 0) {
-        if (out_on_device) { if (cudaMemset(out_doc_tok, 0, (static_cast<size_t>(n_docs) + 1) * 4) != cudaSuccess) return -1; }
+        if (out_on_device) { if (!im.clear_on_device(out_doc_tok, static_cast<size_t>(n_docs) + 1, last_error_)) return -1; }
         else for (uint32_t d = 0; d <= n_docs; ++d) out_doc_tok[d] = 0;
         return 0;
     }
@@ -1101,17 +1138,13 @@ int64_t Engine::encode_batch(const uint8_t* bytes, const uint32_t* doc_off, uint
     if (total < 0) return total;
     if (im.nfc && c->h_status[2] > cap_bytes) { last_error_ = "normalised text is longer than the handle's byte capacity"; return -3; }
     if (static_cast<uint64_t>(total) > out_cap) { last_error_ = "more token ids than the output buffer holds"; return -2; }
-    if (out_on_device) {
-        cudaError_t e = cudaSuccess;
-        if (total) e = cudaMemcpyAsync(out_tokens, c->d_out, static_cast<size_t>(total) * 4, cudaMemcpyDeviceToDevice, c->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(out_doc_tok, c->d_doc_tok, (static_cast<size_t>(n_docs) + 1) * 4, cudaMemcpyDeviceToDevice, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) { last_error_ = std::string("token copy: ") + cudaGetErrorString(e); return -1; }
-        return total;
-    }
+    if (out_on_device)
+        return im.copy_to_device(c, out_tokens, static_cast<size_t>(total), out_doc_tok, static_cast<size_t>(n_docs) + 1, last_error_) ? total : -1;
     if (!im.copy_out(c, out_tokens, static_cast<size_t>(total), out_doc_tok, static_cast<size_t>(n_docs) + 1, last_error_)) return -1;
     return total;
 }
+
+int Engine::order_after(void* stream) { return impl_->order_after(static_cast<cudaStream_t>(stream), last_error_) ? 0 : -1; }
 
 int64_t Engine::measure(const TextPiece* pieces, uint32_t n_pieces, bool batch) {
     Impl& im = *impl_;
@@ -1132,7 +1165,7 @@ int64_t Engine::run_measured(uint64_t len64, uint32_t cap_bytes, uint32_t* dev_t
     cl.c = nullptr;
     cl.tiny = false;
     if (len == 0) {
-        if (cl.batch && dev_doc_tok && cudaMemset(dev_doc_tok, 0, (static_cast<size_t>(cl.docs) + 1) * 4) != cudaSuccess) return -1;
+        if (cl.batch && dev_doc_tok && !im.clear_on_device(dev_doc_tok, static_cast<size_t>(cl.docs) + 1, last_error_)) return -1;
         return cl.total = 0;
     }
     const uint32_t* doc_off = cl.batch ? im.text_off.data() : nullptr;
@@ -1153,12 +1186,7 @@ int64_t Engine::run_measured(uint64_t len64, uint32_t cap_bytes, uint32_t* dev_t
     if (im.nfc && cl.c->h_status[2] > cap_bytes) { last_error_ = "normalised text is longer than the handle's byte capacity"; return -3; }
     if (dev_tokens) {
         if (static_cast<uint64_t>(total) > dev_cap) { last_error_ = "more token ids than the output buffer holds"; return -2; }
-        cudaError_t e = cudaSuccess;
-        if (total) e = cudaMemcpyAsync(dev_tokens, cl.c->d_out, static_cast<size_t>(total) * 4, cudaMemcpyDeviceToDevice, cl.c->stream);
-        if (e == cudaSuccess && dev_doc_tok)
-            e = cudaMemcpyAsync(dev_doc_tok, cl.c->d_doc_tok, (static_cast<size_t>(cl.docs) + 1) * 4, cudaMemcpyDeviceToDevice, cl.c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(cl.c->stream);
-        if (e != cudaSuccess) { last_error_ = std::string("token copy: ") + cudaGetErrorString(e); return -1; }
+        if (!im.copy_to_device(cl.c, dev_tokens, static_cast<size_t>(total), dev_doc_tok, dev_doc_tok ? static_cast<size_t>(cl.docs) + 1 : 0, last_error_)) return -1;
     }
     return cl.total = total;
 }

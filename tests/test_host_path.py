@@ -124,6 +124,30 @@ def test_results_outlive_later_calls(tok, oracles):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("side_stream", (False, True))
+@pytest.mark.parametrize("texts", ("one", "batch", "batch without text"))
+def test_results_on_the_device_wait_for_the_readers_of_their_memory(tok, oracles, side_stream, texts):
+    """A tensor dropped while work that reads it is still queued: the ids that get its block come after that work."""
+    import torch
+    text = _text("ucs2", 3000, 4)
+    want = oracles["llama3"].encode(text.encode())
+    encode = {"one": lambda: (tok.encode_to_device(text), want), "batch": lambda: (tok.encode_batch_to_device([text, ""])[0], want),
+              "batch without text": lambda: (tok.encode_batch_to_device(["", "", ""])[1], np.zeros(4))}[texts]
+    encode()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()                              # so that the block dropped below is the smallest one that fits
+    with torch.cuda.stream(torch.cuda.Stream() if side_stream else torch.cuda.current_stream()):
+        held = torch.full((32768,), 7, dtype=torch.int32, device="cuda")
+        at = held.data_ptr()
+        torch.cuda._sleep(200_000_000)                    # some 0.1 s
+        seen = held + 1
+        del held
+        got, expect = encode()
+        assert at <= got.data_ptr() < at + 4 * 32768      # the block has come back, as the test wants it to
+        assert (seen.cpu() == 8).all() and np.array_equal(got.cpu().numpy(), expect)
+
+
+@pytest.mark.gpu
 def test_refused_inputs(tok):
     for bad in (3, None, [1], ("a",)):
         with pytest.raises(TypeError):
