@@ -283,14 +283,20 @@ struct Engine::Impl {
     std::vector<Slice> slices;
     std::vector<uint32_t> part_slices;   // slices up to the end of each step
     std::vector<uint32_t> text_off;      // batch: where each document begins
-    // a call between put() and take()
+    // The call in steps that is under way: measured and to be encoded (bytes >= 0; `slices` point into the caller's memory),
+    // or encoded and its ids to be taken (total >= 0; they are in c).
     struct Call {
         Ctx* c = nullptr;
         bool tiny = false, batch = false;
-        uint32_t docs = 0, len = 0, cap = 0;
-        int64_t total = -1;
+        uint32_t docs = 0;
+        uint64_t wide = 0;
+        int64_t bytes = -1, total = -1;
     } call;
-    uint64_t call_wide = 0;
+    // Any other call on the handle ends it: that one uses the same buffers, or builds new ones.
+    void end_call() {
+        call = Call();
+        slices.clear();
+    }
 
     Impl() { result_blocks_user(1); }
     ~Impl() {
@@ -1099,6 +1105,7 @@ void Engine::table_bytes(uint64_t* merge, uint64_t* word, uint64_t* other) const
 
 int64_t Engine::encode(const uint8_t* text, uint32_t len, uint32_t cap_bytes, uint32_t* out, uint32_t max_out, bool out_on_device) {
     Impl& im = *impl_;
+    im.end_call();
     cudaSetDevice(im.device);
     if (len == 0) return 0;
     if (!out_on_device && len <= kTinyMaxBytes && im.tiny && !im.nfc) {
@@ -1125,6 +1132,7 @@ int64_t Engine::encode(const uint8_t* text, uint32_t len, uint32_t cap_bytes, ui
 int64_t Engine::encode_batch(const uint8_t* bytes, const uint32_t* doc_off, uint32_t n_docs, uint32_t cap_bytes,
                              uint32_t* out_tokens, uint32_t out_cap, uint32_t* out_doc_tok, bool out_on_device) {
     Impl& im = *impl_;
+    im.end_call();
     cudaSetDevice(im.device);
     const uint32_t len = doc_off[n_docs];
     if (len == 0) {
@@ -1148,25 +1156,36 @@ int Engine::order_after(void* stream) { return impl_->order_after(static_cast<cu
 
 int64_t Engine::measure(const TextPiece* pieces, uint32_t n_pieces, bool batch) {
     Impl& im = *impl_;
-    im.call = Impl::Call();
+    im.end_call();
+    uint64_t total = 0, wide = 0;
+    if (!im.measure(pieces, n_pieces, batch, &total, &wide)) { im.end_call(); last_error_ = "a character has no UTF-8 form"; return -1; }
     im.call.batch = batch;
     im.call.docs = batch ? n_pieces : 1;
-    uint64_t total = 0;
-    if (!im.measure(pieces, n_pieces, batch, &total, &im.call_wide)) return -1;
-    return static_cast<int64_t>(std::min<uint64_t>(total, INT64_MAX));
+    im.call.wide = wide;
+    return im.call.bytes = static_cast<int64_t>(std::min<uint64_t>(total, INT64_MAX));
 }
 
-int64_t Engine::run_measured(uint64_t len64, uint32_t cap_bytes, uint32_t* dev_tokens, uint32_t dev_cap, uint32_t* dev_doc_tok) {
+int64_t Engine::run_measured(uint64_t bytes, uint32_t cap_bytes, uint32_t* dev_tokens, uint32_t dev_cap, uint32_t* dev_doc_tok) {
+    Impl& im = *impl_;
+    // (the pieces are written by the places measure() found for them, into buffers made for `bytes`)
+    if (im.call.bytes < 0 || static_cast<uint64_t>(im.call.bytes) != bytes || bytes > 0xFFFFFF00ull) { last_error_ = "no measured text of that length"; return -1; }
+    const int64_t total = encode_slices(static_cast<uint32_t>(bytes), cap_bytes, dev_tokens, dev_cap, dev_doc_tok);
+    if (total == -2) return total;           // the same text may follow with more room
+    if (total < 0) { im.end_call(); return total; }
+    im.call.bytes = -1;
+    im.slices.clear();
+    return im.call.total = total;
+}
+
+int64_t Engine::encode_slices(uint32_t len, uint32_t cap_bytes, uint32_t* dev_tokens, uint32_t dev_cap, uint32_t* dev_doc_tok) {
     Impl& im = *impl_;
     Impl::Call& cl = im.call;
     cudaSetDevice(im.device);
-    const uint32_t len = static_cast<uint32_t>(len64);
-    cl.total = -1;
     cl.c = nullptr;
     cl.tiny = false;
     if (len == 0) {
         if (cl.batch && dev_doc_tok && !im.clear_on_device(dev_doc_tok, static_cast<size_t>(cl.docs) + 1, last_error_)) return -1;
-        return cl.total = 0;
+        return 0;
     }
     const uint32_t* doc_off = cl.batch ? im.text_off.data() : nullptr;
     cl.c = im.ctx_for(cl.batch, len, cl.docs, cap_bytes, last_error_);
@@ -1176,11 +1195,11 @@ int64_t Engine::run_measured(uint64_t len64, uint32_t cap_bytes, uint32_t* dev_t
         const int64_t r = im.launch_tiny_graph(cl.c, len, last_error_);
         if (r != Impl::kNoCtx) {
             cl.tiny = true;
-            return cl.total = r;
+            return r;
         }
     }
-    if (!im.stage_slices(cl.c, len, im.call_wide, doc_off, cl.docs, last_error_)) return -1;
-    int64_t total = im.run_staged(cl.c, cl.batch, cl.c->h_text, len, doc_off, cl.docs, cap_bytes, last_error_);
+    if (!im.stage_slices(cl.c, len, cl.wide, doc_off, cl.docs, last_error_)) return -1;
+    const int64_t total = im.run_staged(cl.c, cl.batch, cl.c->h_text, len, doc_off, cl.docs, cap_bytes, last_error_);
     if (total == Impl::kNoCtx) return cl.batch ? -4 : -1;
     if (total < 0) return total;
     if (im.nfc && cl.c->h_status[2] > cap_bytes) { last_error_ = "normalised text is longer than the handle's byte capacity"; return -3; }
@@ -1188,7 +1207,7 @@ int64_t Engine::run_measured(uint64_t len64, uint32_t cap_bytes, uint32_t* dev_t
         if (static_cast<uint64_t>(total) > dev_cap) { last_error_ = "more token ids than the output buffer holds"; return -2; }
         if (!im.copy_to_device(cl.c, dev_tokens, static_cast<size_t>(total), dev_doc_tok, dev_doc_tok ? static_cast<size_t>(cl.docs) + 1 : 0, last_error_)) return -1;
     }
-    return cl.total = total;
+    return total;
 }
 
 int Engine::take_ids(uint32_t* out, uint32_t* out_doc_tok) {
@@ -1196,8 +1215,9 @@ int Engine::take_ids(uint32_t* out, uint32_t* out_doc_tok) {
     Impl::Call& cl = im.call;
     if (cl.total < 0) { last_error_ = "no finished call to take the ids of"; return -1; }
     const size_t total = static_cast<size_t>(cl.total), doc_words = cl.batch ? static_cast<size_t>(cl.docs) + 1 : 0;
+    if ((total && !out) || (doc_words && !out_doc_tok)) { last_error_ = "no place for the ids or the offsets"; return -1; }
     cl.total = -1;
-    if (!cl.c) { std::memset(out_doc_tok, 0, doc_words * 4); return 0; }
+    if (!cl.c) { if (doc_words) std::memset(out_doc_tok, 0, doc_words * 4); return 0; }
     if (cl.tiny) { std::memcpy(out, cl.c->h_tiny_out, total * 4); return 0; }
     if (!total && !doc_words) return 0;
     cudaSetDevice(im.device);
@@ -1206,6 +1226,7 @@ int Engine::take_ids(uint32_t* out, uint32_t* out_doc_tok) {
 
 int Engine::stage(const uint8_t* bytes, uint32_t len, const uint32_t* doc_off, uint32_t n_docs, uint32_t cap_bytes) {
     Impl& im = *impl_;
+    im.end_call();
     cudaSetDevice(im.device);
     const bool batch_mode = doc_off != nullptr;
     Ctx* c = im.ctx_for(batch_mode, len, batch_mode ? n_docs : 1, cap_bytes, last_error_);
@@ -1218,6 +1239,7 @@ int Engine::stage(const uint8_t* bytes, uint32_t len, const uint32_t* doc_off, u
 
 int64_t Engine::replay_staged(float* ms_out) {
     Impl& im = *impl_;
+    im.end_call();
     cudaSetDevice(im.device);
     if (!im.staged) { last_error_ = "nothing staged"; return -1; }
     return im.replay(im.staged, true, ms_out, last_error_);
@@ -1225,6 +1247,7 @@ int64_t Engine::replay_staged(float* ms_out) {
 
 int64_t Engine::profile_staged(float* ms_out) {
     Impl& im = *impl_;
+    im.end_call();
     cudaSetDevice(im.device);
     Ctx* c = im.staged;
     if (!c) { last_error_ = "nothing staged"; return -1; }

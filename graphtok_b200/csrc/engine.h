@@ -38,14 +38,16 @@ public:
     // themselves once its size is known:
     //   measure       the text's UTF-8 bytes; -1 where a character has no UTF-8 form.  With `batch` each piece is a document.
     //   run_measured  stages the pieces (which must still be in place) and replays; ids stay inside, or go to `dev_tokens`
-    //                 (and `dev_doc_tok`, n_docs + 1 offsets) on the device.  `bytes` is what measure returned.
-    //   take_ids      ids and offsets of the finished call to host memory; 0 or -1.
+    //                 (and `dev_doc_tok`, n_docs + 1 offsets) on the device.  `bytes` is what measure returned; -1 for anything
+    //                 else, and when no measured text is there: a text is encoded once, but for a -2, which more room may follow.
+    //   take_ids      ids and offsets of the finished call to host memory; 0 or -1.  Once.
+    // Another encode, stage or replay ends the call.
     int64_t measure(const TextPiece* pieces, uint32_t n_pieces, bool batch);
     int64_t run_measured(uint64_t bytes, uint32_t cap_bytes, uint32_t* dev_tokens, uint32_t dev_cap, uint32_t* dev_doc_tok);
     int take_ids(uint32_t* out, uint32_t* out_doc_tok);
 
-    // Decoding in steps: a page-locked buffer for `n` ids that decode_run then need not copy (optional), the decode
-    // itself, and the bytes it gave to host memory (0 or -1).
+    // Decoding in steps: a page-locked buffer for `n` ids that decode_run then need not copy (optional; it is there until the
+    // next decode call on the handle), the decode itself, and the bytes it gave to host memory (0 or -1).
     uint32_t* decode_room(uint32_t n);
     int64_t decode_run(const uint32_t* ids, uint32_t n, uint64_t max_out, uint64_t* need, float* kernel_ms);
     int take_bytes(uint8_t* out);
@@ -90,6 +92,7 @@ public:
 
 private:
     Engine() = default;
+    int64_t encode_slices(uint32_t len, uint32_t cap_bytes, uint32_t* dev_tokens, uint32_t dev_cap, uint32_t* dev_doc_tok);
     bool decode_ctx(uint32_t n, uint64_t want);
     struct Impl;
     std::unique_ptr<Impl> impl_;

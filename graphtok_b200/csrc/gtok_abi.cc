@@ -358,7 +358,10 @@ int64_t gtok_x_measure(void* handle, const gtok_x_piece* pieces, uint32_t n_piec
     if (!handle || (!pieces && n_pieces)) return -1;
     static_assert(sizeof(gtok_x_piece) == sizeof(gtok::TextPiece), "the same layout on both sides of the boundary");
     try {
-        return static_cast<Handle*>(handle)->engine->measure(reinterpret_cast<const gtok::TextPiece*>(pieces), n_pieces, batch != 0);
+        Handle* h = static_cast<Handle*>(handle);
+        const int64_t r = h->engine->measure(reinterpret_cast<const gtok::TextPiece*>(pieces), n_pieces, batch != 0);
+        if (r < 0) g_last_error = h->engine->last_error();
+        return r;
     } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
 }
 

@@ -164,14 +164,17 @@ int64_t gtok_x_decode(void* handle, const uint32_t* ids, uint32_t n, uint8_t* ou
 
 /* The encode and decode calls in steps, for bindings that hold text in pieces (a list of strings) and make
  * the result's memory themselves once its size is known.  A handle takes one call at a time: measure, encode
- * and take belong together, with nothing else on the handle in between.
+ * and take belong together; any other call that encodes, stages or replays on the handle ends them, and the
+ * step that would have come next answers -1.
  *   gtok_x_measure         UTF-8 bytes of the pieces, which are the documents of a batch or the parts of one
  *                          text; -1 where a character has no UTF-8 form (a surrogate)
  *   gtok_x_encode_measured encodes them (they must still be in place) and returns the id count; return codes as
- *                          gtok_encode / gtok_encode_batch.  With out_dev the ids (and with out_doc_dev the
+ *                          gtok_encode / gtok_encode_batch.  `bytes` is what gtok_x_measure returned (-1 for anything
+ *                          else); after -2 the same text may follow with more room, else once.  With out_dev the ids (and with out_doc_dev the
  *                          n_pieces + 1 token offsets of a batch) go to device memory, else gtok_x_take_ids
  *                          copies them to host memory (directly where that is page-locked)
- *   gtok_x_decode_room     a page-locked buffer for n ids; ids put there need no further copy.  Optional
+ *   gtok_x_decode_room     a page-locked buffer for n ids; ids put there need no further copy.  Optional; the
+ *                          buffer is the handle's, until its next decoding call
  *   gtok_x_decode_run      ids -> bytes, which gtok_x_take_bytes copies to host memory; returns their number
  *   gtok_x_block_get       page-locked memory for a result, from a bounded pool shared by all handles and
  *                          threads; NULL when the pool is exhausted (use ordinary memory then)

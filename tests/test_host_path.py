@@ -167,3 +167,51 @@ def test_refused_inputs(tok):
     for ids in ([72, 105], [True, 3], np.array([[72, 105]], dtype=np.uint16), np.arange(40)[::2], np.arange(9, dtype=np.int32), (7, 8), []):
         assert tok.decode_bytes(ids) == tok._g.decode(np.asarray(ids).astype(np.uint32).reshape(-1), want_ms=True)[0]
     assert tok.encode_numpy("still works").size > 0
+
+
+class Piece(ctypes.Structure):
+    _fields_ = [("data", ctypes.c_void_p), ("units", ctypes.c_uint64), ("kind", ctypes.c_uint32)]
+
+
+@pytest.mark.gpu
+def test_steps_out_of_order_are_refused(oracles):
+    """gtok_x_measure, gtok_x_encode_measured, gtok_x_take_ids: a length that was not measured, a step twice, a step whose call
+    another one has ended."""
+    from graphtok_b200 import GTok
+    g = GTok(tiny_vocab("llama3"))
+    lib, h = g.lib, ctypes.c_void_p(g.handle)
+    for name, types in (("gtok_x_measure", [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_int32]),
+                        ("gtok_x_encode_measured", [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p])):
+        getattr(lib, name).restype, getattr(lib, name).argtypes = ctypes.c_int64, types
+    lib.gtok_x_take_ids.restype, lib.gtok_x_take_ids.argtypes = ctypes.c_int32, [ctypes.c_void_p] * 3
+    for size in (100, 50000):                    # the single-block route and the other
+        text = _text("ascii", size, 9).encode()
+        want = oracles["llama3"].encode(text)
+        keep = ctypes.create_string_buffer(text)
+        piece = Piece(ctypes.addressof(keep), len(text), 1)
+        out = np.zeros(len(text) + 16, dtype=np.uint32)
+
+        def measure():
+            return lib.gtok_x_measure(h, ctypes.byref(piece), 1, 0)
+
+        def encode(n):
+            return lib.gtok_x_encode_measured(h, n, None, 0, None)
+
+        def take():
+            return lib.gtok_x_take_ids(h, out.ctypes.data, None)
+        assert measure() == len(text)
+        assert encode(len(text) - 1) == encode(len(text) + 1) == encode(0) == -1
+        assert take() == -1                      # nothing encoded yet
+        assert encode(len(text)) == want.size and encode(len(text)) == -1
+        assert lib.gtok_x_take_ids(h, None, None) == -1
+        assert take() == 0 and np.array_equal(out[:want.size], want) and take() == -1
+        for other in (lambda: g.encode(b"other"), lambda: g.encode_batch(b"other", [0, 2, 5]), lambda: g.stage(b"other"), lambda: (g.stage(b"other"), g.replay())):
+            assert measure() == len(text)
+            other()
+            assert encode(len(text)) == -1
+            g.stage(b"first")
+            assert measure() == len(text) and encode(len(text)) == want.size
+            other()
+            assert take() == -1
+    assert "finished" in lib.gtok_x_last_error().decode()
+    g.close()
