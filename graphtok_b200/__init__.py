@@ -127,6 +127,7 @@ class GTok:
         if not self.handle:
             raise GTokError("gtok_create failed: %s" % self.lib.gtok_x_last_error().decode("utf-8", "replace"))
         self.max_bytes = max(4096, int(max_bytes))
+        self.host.users(1)
 
     def set_max_bytes(self, max_bytes):
         """Raises the handle's byte cap in place (tables stay; the context grows when next needed)."""
@@ -137,6 +138,7 @@ class GTok:
         if getattr(self, "handle", None):
             self.lib.gtok_destroy(self.handle)
             self.handle = None
+            self.host.users(-1)
 
     def __del__(self):
         try:
@@ -168,7 +170,8 @@ class GTok:
             n = self.lib.gtok_encode_batch(self.handle, blob, offsets.ctypes.data, n_docs, out.ctypes.data, out.size, doc.ctypes.data)
         if n < 0:
             self._fail("gtok_encode_batch", n)
-        return out[:n], doc
+        out.resize(n, refcheck=False)
+        return out, doc
 
     # ---- measurement -----------------------------------------------------
     def stage(self, blob, offsets=None):

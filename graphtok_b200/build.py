@@ -24,7 +24,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "--shared",
     "-Xlinker", "--version-script=" + os.path.join(CSRC, "gtok.map"),
 ]
-SOURCES = ["encode_kernels.cu", "tiny_kernel.cu", "engine.cu", "gtok_abi.cc", "vocab_host.cc", "tables_build.cc", "nfc_host.cc", "host_text.cc", "result_blocks.cc"]
+SOURCES = ["encode_kernels.cu", "tiny_kernel.cu", "engine.cu", "gtok_abi.cc", "vocab_host.cc", "tables_build.cc", "nfc_host.cc", "host_text.cc"]
 
 
 def _newer(target, deps):
@@ -104,7 +104,7 @@ def build_host(force=False):
     """The CPython extension between the Python classes and libgtok.so; None where it cannot be built, and the classes
     then go by ctypes (ctypes_host.py)."""
     src = os.path.join(HERE, "pyhost", "host_module.cc")
-    if not force and not _newer(HOST, [src, os.path.join(HERE, "..", "include", "gtok.h")]):
+    if not force and not _newer(HOST, [src, os.path.join(HERE, "pyhost", "result_memory.h"), os.path.join(HERE, "..", "include", "gtok.h")]):
         return HOST
     if os.path.exists(HOST):
         os.remove(HOST)          # an outdated one must not be loaded

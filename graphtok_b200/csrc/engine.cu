@@ -18,7 +18,6 @@
 #include "encode_kernels.h"
 #include "host_text.h"
 #include "nfc_host.h"
-#include "result_blocks.h"
 #include "tables_build.h"
 #include "unicode_class_table.h"
 #include "unicode_wide_table.h"
@@ -298,9 +297,7 @@ struct Engine::Impl {
         slices.clear();
     }
 
-    Impl() { result_blocks_user(1); }
     ~Impl() {
-        result_blocks_user(-1);
         single.reset();
         batch.reset();
         dec.reset();

@@ -14,7 +14,6 @@
 #include "device_tables.h"
 #include "encode_kernels.h"
 #include "engine.h"
-#include "result_blocks.h"
 #include "shard_plan.h"
 
 namespace {
@@ -417,13 +416,6 @@ int32_t gtok_x_take_bytes(void* handle, uint8_t* out) {
         if (r < 0) g_last_error = h->engine->last_error();
         return r;
     } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
-}
-
-void* gtok_x_block_get(uint64_t bytes) {
-    try { return gtok::result_block_get(static_cast<size_t>(bytes)); } catch (...) { return nullptr; }
-}
-void gtok_x_block_put(void* block) {
-    if (block) gtok::result_block_put(block);
 }
 
 int32_t gtok_x_plan_chunks(void* handle, const uint8_t* text, uint64_t len, uint32_t n_parts, uint64_t* out_offsets) {

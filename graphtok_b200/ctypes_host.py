@@ -36,6 +36,9 @@ class CtypesHost:
     def __init__(self, lib):
         self.lib = lib
 
+    def users(self, change):
+        pass                     # nothing is kept between calls
+
     def _grow(self, handle, n_bytes):
         # doubled until a text of that many bytes fits even if NFC lengthens it (at most threefold)
         cap = int(self.lib.gtok_x_set_max_bytes(handle, 0))

@@ -10,20 +10,22 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #define NPY_NO_DEPRECATED_API NPY_1_7_API_VERSION
+#define NPY_TARGET_VERSION NPY_1_22_API_VERSION
 #include <numpy/arrayobject.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
 #include "../../include/gtok.h"
+#include "result_memory.h"
 
 namespace {
 
-// Results from this size on come in page-locked blocks (below it the copy out of the handle's own page-locked
-// buffer takes less than a transfer of its own would).
-constexpr uint64_t kBlockBytes = 256 << 10;
+// Results from this size on are copied out with the interpreter lock let go.
+constexpr uint64_t kLargeBytes = 256 << 10;
 
 // The library's calls by address.
 struct Lib {
@@ -34,14 +36,12 @@ struct Lib {
     decltype(&gtok_x_decode_room) decode_room;
     decltype(&gtok_x_decode_run) decode_run;
     decltype(&gtok_x_take_bytes) take_bytes;
-    decltype(&gtok_x_block_get) block_get;
-    decltype(&gtok_x_block_put) block_put;
 } lib;
 bool bound = false;
 struct Need { const char* name; void* at; };
 #define GTOK_NEED(f) {"gtok_x_" #f, &lib.f}
 const Need kNeeds[] = {GTOK_NEED(set_max_bytes), GTOK_NEED(measure), GTOK_NEED(encode_measured), GTOK_NEED(take_ids), GTOK_NEED(decode_room),
-                       GTOK_NEED(decode_run), GTOK_NEED(take_bytes), GTOK_NEED(block_get), GTOK_NEED(block_put)};
+                       GTOK_NEED(decode_run), GTOK_NEED(take_bytes)};
 
 // bind(address): address(name) -> where that call of gtok.h is in the loaded library.
 PyObject* py_bind(PyObject*, PyObject* address) {
@@ -122,21 +122,30 @@ void grow_cap(void* h, int64_t bytes) {
     lib.set_max_bytes(h, static_cast<uint32_t>(std::min<uint64_t>(cap, 0xFFFFFFFFull)));
 }
 
-void release_block(PyObject* capsule) { lib.block_put(PyCapsule_GetPointer(capsule, nullptr)); }
+// numpy's memory functions over result_memory.h; an array keeps the handler it was made with.
+void* mem_get(void*, size_t size) { return result_memory::get(size); }
+void* mem_zeroed(void*, size_t n, size_t each) { return std::calloc(n, each); }
+void* mem_resize(void*, void* p, size_t size) { return std::realloc(p, size); }
+void mem_put(void*, void* p, size_t) { result_memory::put(p); }
+PyDataMem_Handler kMemory = {"graphtok_results", 1, {nullptr, mem_get, mem_zeroed, mem_resize, mem_put}};
+PyObject* memory = nullptr;      // its capsule
 
-// An array for `n` ids.
+// An array for `n` ids that owns its memory.
 PyObject* new_ids(int64_t n) {
     npy_intp dim = static_cast<npy_intp>(n);
-    if (static_cast<uint64_t>(n) * 4 >= kBlockBytes) {
-        if (void* p = lib.block_get(static_cast<uint64_t>(n) * 4)) {
-            PyObject* a = PyArray_SimpleNewFromData(1, &dim, NPY_UINT32, p);
-            PyObject* c = a ? PyCapsule_New(p, nullptr, release_block) : nullptr;
-            if (!c) { Py_XDECREF(a); lib.block_put(p); return nullptr; }
-            if (PyArray_SetBaseObject(reinterpret_cast<PyArrayObject*>(a), c) < 0) { Py_DECREF(a); return nullptr; }     // (the capsule is gone either way)
-            return a;
-        }
-    }
-    return PyArray_SimpleNew(1, &dim, NPY_UINT32);
+    if (static_cast<uint64_t>(n) * 4 < result_memory::kLeast) return PyArray_SimpleNew(1, &dim, NPY_UINT32);
+    PyObject* usual = PyDataMem_GetHandler();
+    if (!usual) return nullptr;
+    if (usual != PyDataMem_DefaultHandler) { Py_DECREF(usual); return PyArray_SimpleNew(1, &dim, NPY_UINT32); }     // the program's own choice
+    Py_DECREF(usual);
+    usual = PyDataMem_SetHandler(memory);
+    if (!usual) return nullptr;
+    PyObject* ids = PyArray_SimpleNew(1, &dim, NPY_UINT32);
+    PyObject* mine = PyDataMem_SetHandler(usual);
+    Py_DECREF(usual);
+    if (!mine) { Py_XDECREF(ids); return nullptr; }
+    Py_DECREF(mine);
+    return ids;
 }
 uint32_t* data_of(PyObject* a) { return static_cast<uint32_t*>(PyArray_DATA(reinterpret_cast<PyArrayObject*>(a))); }
 
@@ -180,7 +189,7 @@ PyObject* py_encode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     PyObject* ids = new_ids(o.ids);
     if (!ids) return nullptr;
     int r;
-    if (static_cast<uint64_t>(o.ids) * 4 < kBlockBytes) {
+    if (static_cast<uint64_t>(o.ids) * 4 < kLargeBytes) {
         r = lib.take_ids(h, data_of(ids), nullptr);
     } else {
         Py_BEGIN_ALLOW_THREADS
@@ -343,7 +352,16 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return bytes;
 }
 
+// users(change): +1 for a tokenizer that is opened, -1 when it is closed
+PyObject* py_users(PyObject*, PyObject* change) {
+    const long v = PyLong_AsLong(change);
+    if (v == -1 && PyErr_Occurred()) return nullptr;
+    result_memory::users(static_cast<int>(v));
+    Py_RETURN_NONE;
+}
+
 PyMethodDef kMethods[] = {
+    {"users", py_users, METH_O, "users(change): tokenizers opened (+1) or closed (-1); memory of dropped results is kept while one is open"},
     {"bind", py_bind, METH_O, "bind(address): address(name) -> address of that call of gtok.h in the loaded library"},
     {"encode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode)), METH_FASTCALL, "encode(handle, text, grow) -> uint32 array, or an error code"},
     {"encode_batch", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode_batch)), METH_FASTCALL,
@@ -359,5 +377,6 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "Python objects to and fr
 
 PyMODINIT_FUNC PyInit__host(void) {
     import_array();
-    return PyModule_Create(&kModule);
+    memory = PyCapsule_New(&kMemory, "mem_handler", nullptr);
+    return memory ? PyModule_Create(&kModule) : nullptr;
 }

@@ -176,8 +176,6 @@ int64_t gtok_x_decode(void* handle, const uint32_t* ids, uint32_t n, uint8_t* ou
  *   gtok_x_decode_room     a page-locked buffer for n ids; ids put there need no further copy.  Optional; the
  *                          buffer is the handle's, until its next decoding call
  *   gtok_x_decode_run      ids -> bytes, which gtok_x_take_bytes copies to host memory; returns their number
- *   gtok_x_block_get       page-locked memory for a result, from a bounded pool shared by all handles and
- *                          threads; NULL when the pool is exhausted (use ordinary memory then)
  */
 typedef struct {
     const void* data;
@@ -190,8 +188,6 @@ int32_t gtok_x_take_ids(void* handle, uint32_t* out, uint32_t* out_doc_offsets);
 uint32_t* gtok_x_decode_room(void* handle, uint32_t n);
 int64_t gtok_x_decode_run(void* handle, const uint32_t* ids, uint32_t n);
 int32_t gtok_x_take_bytes(void* handle, uint8_t* out);
-void* gtok_x_block_get(uint64_t bytes);
-void gtok_x_block_put(void* block);
 
 /* Partitioning over the GPUs of one box (no counterpart in the reference, which is
  * single-GPU).  gtok_x_plan_chunks cuts one document into n_parts pieces at

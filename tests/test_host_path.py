@@ -80,7 +80,7 @@ def tok(request):
 
 
 # sizes: single-block route and its limit, one copy step and several, the size from which characters are shared among
-# threads, results below and above the size of a page-locked block
+# threads, results below and above the size from which the memory of dropped ones is kept
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", list(WIDTH))
 @pytest.mark.parametrize("n", [0, 1, 33, 2047, 2049, 40000, 70001, 400003])
@@ -111,7 +111,7 @@ def test_batch_of_mixed_objects(tok, oracles, docs, longest):
 
 @pytest.mark.gpu
 def test_results_outlive_later_calls(tok, oracles):
-    """More large results at once than there are page-locked blocks: each stays as it was."""
+    """Large results held at once, and a view of a dropped one: each stays as it was."""
     texts = [_text("ucs2", 120000, i) for i in range(9)]
     got = [tok.encode_numpy(t) for t in texts]
     for t, g in zip(texts, got):
