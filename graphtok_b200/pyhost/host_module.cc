@@ -17,6 +17,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "../../include/gtok.h"
@@ -70,11 +71,26 @@ struct Texts {
     std::vector<Py_buffer> buffers;
     gtok_x_piece one;
     ~Texts() {
-        for (PyObject* o : kept) Py_DECREF(o);
+        for (PyObject* o : kept) Py_XDECREF(o);
         for (Py_buffer& b : buffers) PyBuffer_Release(&b);
     }
-    // False with an exception set: neither str nor bytes-like.
-    bool place(PyObject* o, gtok_x_piece* p) {
+    // False with an exception set: neither str nor bytes-like, or no memory to note it down.
+    bool place(PyObject* o, gtok_x_piece* p) noexcept {
+        try { return find(o, p); } catch (const std::bad_alloc&) { PyErr_NoMemory(); return false; }
+    }
+    // The same for the texts of a tuple, as `pieces`.
+    bool place_all(PyObject* tuple) noexcept {
+        const Py_ssize_t n = PyTuple_GET_SIZE(tuple);
+        try {
+            pieces.resize(static_cast<size_t>(n));
+        } catch (const std::exception&) { PyErr_NoMemory(); return false; }
+        for (Py_ssize_t i = 0; i < n; ++i)
+            if (!place(PyTuple_GET_ITEM(tuple, i), &pieces[static_cast<size_t>(i)])) return false;
+        return true;
+    }
+
+private:
+    bool find(PyObject* o, gtok_x_piece* p) {
         if (PyUnicode_CheckExact(o)) {
             p->data = PyUnicode_DATA(o);
             p->units = static_cast<uint64_t>(PyUnicode_GET_LENGTH(o));
@@ -89,22 +105,23 @@ struct Texts {
             return true;
         }
         if (PyByteArray_CheckExact(o) || PyMemoryView_Check(o)) {
-            Py_buffer b;
-            if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) == 0) {
-                buffers.push_back(b);
-                p->data = b.buf;
-                p->units = static_cast<uint64_t>(b.len);
+            buffers.emplace_back();
+            if (PyObject_GetBuffer(o, &buffers.back(), PyBUF_SIMPLE) == 0) {
+                p->data = buffers.back().buf;
+                p->units = static_cast<uint64_t>(buffers.back().len);
                 p->kind = 1;
                 return true;
             }
+            buffers.pop_back();
             PyErr_Clear();          // a view with gaps: its bytes below
         }
+        kept.push_back(nullptr);
         PyObject* made = nullptr;
         if (PyUnicode_Check(o)) made = PyObject_CallMethod(o, "encode", "s", "utf-8");
         else if (PyBytes_Check(o) || PyByteArray_Check(o) || PyMemoryView_Check(o)) made = PyObject_Bytes(o);
         else { PyErr_SetString(PyExc_TypeError, "text must be str or bytes"); return false; }
         if (!made) return false;
-        kept.push_back(made);
+        kept.back() = made;
         if (!PyBytes_Check(made)) { PyErr_SetString(PyExc_TypeError, "text must be str or bytes"); return false; }
         p->data = PyBytes_AS_STRING(made);
         p->units = static_cast<uint64_t>(PyBytes_GET_SIZE(made));
@@ -200,21 +217,11 @@ PyObject* py_encode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return ids;
 }
 
-// The texts of a sequence as pieces.  `seq` (from PySequence_Fast on a list or tuple that this call alone holds)
-bool place_all(Texts& t, PyObject* seq) {
-    const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
-    PyObject** items = PySequence_Fast_ITEMS(seq);
-    t.pieces.resize(static_cast<size_t>(n));
-    for (Py_ssize_t i = 0; i < n; ++i)
-        if (!t.place(items[i], &t.pieces[static_cast<size_t>(i)])) return false;
-    return true;
-}
-
 // encode_batch(handle, texts (a tuple, at least one), grow) -> (uint32 ids, uint32 offsets)
 PyObject* py_encode_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (nargs != 3 || !PyTuple_CheckExact(args[1])) { PyErr_SetString(PyExc_TypeError, "encode_batch(handle, tuple of texts, grow)"); return nullptr; }
     Texts t;
-    if (!place_all(t, args[1])) return nullptr;
+    if (!t.place_all(args[1])) return nullptr;
     void* h = handle_of(args[0]);
     if (!h) return PyLong_FromLong(-1);
     const Outcome o = encode_texts(h, t.pieces.data(), static_cast<uint32_t>(t.pieces.size()), true, args[2] == Py_True);
@@ -239,7 +246,7 @@ PyObject* py_encode_to_device(PyObject*, PyObject* const* args, Py_ssize_t nargs
     if (nargs != 4) { PyErr_SetString(PyExc_TypeError, "encode_to_device(handle, text or tuple, grow, make)"); return nullptr; }
     const bool batch = PyTuple_CheckExact(args[1]);
     Texts t;
-    if (batch ? !place_all(t, args[1]) : !t.place(args[1], &t.one)) return nullptr;
+    if (batch ? !t.place_all(args[1]) : !t.place(args[1], &t.one)) return nullptr;
     void* h = handle_of(args[0]);
     if (!h) return PyLong_FromLong(-1);
     const gtok_x_piece* p = batch ? t.pieces.data() : &t.one;
