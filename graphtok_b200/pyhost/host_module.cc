@@ -1,8 +1,8 @@
 // graphtok_b200._host: what stands between a Python object and libgtok's calls in steps (gtok_x_measure and
 // what follows it in gtok.h).
 //
-// The library takes text where Python keeps it (a str's own characters, a bytes object's bytes, the strings of a
-// list one by one) and writes ids and bytes to the object that is returned, so a call makes no intermediate
+// The library takes text where Python keeps it (a str's own characters, a bytes object's bytes, those of a list
+// one by one) and writes ids and bytes to the object that is returned, so a call makes no intermediate
 // Python object and no copy that the transfer to or from the GPU does not need.  Every function takes the
 // handle as an integer and answers an error of the library with its (negative) code as an int.
 // The module is not linked against the library: bind() takes the calls' addresses from whoever has loaded it, so
@@ -68,11 +68,9 @@ void* handle_of(PyObject* o) { return bound && PyLong_CheckExact(o) ? PyLong_AsV
 struct Texts {
     std::vector<gtok_x_piece> pieces;
     std::vector<PyObject*> kept;
-    std::vector<Py_buffer> buffers;
     gtok_x_piece one;
     ~Texts() {
         for (PyObject* o : kept) Py_XDECREF(o);
-        for (Py_buffer& b : buffers) PyBuffer_Release(&b);
     }
     // False with an exception set: neither str nor bytes-like, or no memory to note it down.
     bool place(PyObject* o, gtok_x_piece* p) noexcept {
@@ -104,19 +102,10 @@ private:
             p->kind = 1;
             return true;
         }
-        if (PyByteArray_CheckExact(o) || PyMemoryView_Check(o)) {
-            buffers.emplace_back();
-            if (PyObject_GetBuffer(o, &buffers.back(), PyBUF_SIMPLE) == 0) {
-                p->data = buffers.back().buf;
-                p->units = static_cast<uint64_t>(buffers.back().len);
-                p->kind = 1;
-                return true;
-            }
-            buffers.pop_back();
-            PyErr_Clear();          // a view with gaps: its bytes below
-        }
         kept.push_back(nullptr);
         PyObject* made = nullptr;
+        // (a bytearray or a view is taken as it is now: while the library works the interpreter lock is let go, and other threads
+        // may write to it or resize it)
         if (PyUnicode_Check(o)) made = PyObject_CallMethod(o, "encode", "s", "utf-8");
         else if (PyBytes_Check(o) || PyByteArray_Check(o) || PyMemoryView_Check(o)) made = PyObject_Bytes(o);
         else { PyErr_SetString(PyExc_TypeError, "text must be str or bytes"); return false; }

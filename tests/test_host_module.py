@@ -39,3 +39,23 @@ for call in (lambda: host.encode_batch(0, texts, False), lambda: host.encode_to_
     except MemoryError:
         print("refused", end=" ")
 """) == "refused refused"
+
+
+def test_a_buffer_that_changes_during_the_call(built):
+    """A bytearray, alone, in a batch and under a view: its bytes of before the call, and free to be resized meanwhile."""
+    assert extension("""
+seen = []
+def measure(handle, pieces, n, batch):
+    buf.extend(b"more" * 100)                            # BufferError while somebody holds the buffer
+    buf[:5] = b"other"
+    at, units = ctypes.c_void_p.from_address(pieces).value, ctypes.c_uint64.from_address(pieces + 8).value
+    seen.append(ctypes.string_at(at, units))
+    return -1
+stand_in(measure=measure)
+for form in (lambda b: host.encode(1, b, False), lambda b: host.encode_batch(1, (b,), False), lambda b: host.encode_to_device(1, b, False, None)):
+    buf = bytearray(b"first and the rest")
+    form(buf)
+buf, whole = bytearray(b"another"), bytearray(b"under a view")
+host.encode(1, memoryview(whole), False)
+print(seen == [b"first and the rest"] * 3 + [b"under a view"], end="")
+""") == "True"
