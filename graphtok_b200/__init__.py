@@ -222,13 +222,13 @@ class GTok:
         """ids -> the bytes they spell, on the device (gtok_x_decode).  `out`: optional uint8 numpy
         buffer to decode into (a page-locked one is written directly); returns bytes, or with
         `want_ms` (bytes, CUDA-event ms of the decode graph)."""
+        ids = np.ascontiguousarray(ids, dtype=np.uint32)
         if out is None and not want_ms:
             data = self.host.decode(self.handle, ids)
             if data.__class__ is bytes:
                 return data
             if data is not None:
                 self._fail("gtok_x_decode", data)
-        ids = np.ascontiguousarray(ids, dtype=np.uint32)
         need = ctypes.c_uint64(0)
         ms = ctypes.c_float(0.0)
         buf = out if out is not None else np.empty(16 * ids.size + 1024, dtype=np.uint8)

@@ -1,5 +1,6 @@
 """The CPython extension by itself (no GPU): what it does with its arguments before and while the library works, the library's
 calls stood in for by functions of the test where they are reached.  Each test in a process of its own."""
+import numpy as np
 import pytest
 
 from test_build_and_load import child
@@ -59,3 +60,22 @@ buf, whole = bytearray(b"another"), bytearray(b"under a view")
 host.encode(1, memoryview(whole), False)
 print(seen == [b"first and the rest"] * 3 + [b"under a view"], end="")
 """) == "True"
+
+
+def test_ids_of_other_types_in_gtok_decode():
+    """GTok.decode converts to uint32 as numpy does, whatever takes the ids then (Tokenizer.decode checks their range first)."""
+    from graphtok_b200 import GTok
+    got = []
+
+    class Host:
+        def decode(self, handle, ids):
+            got.append(ids)
+            return b"text"
+    g = GTok.__new__(GTok)
+    g.handle, g.host = None, Host()
+    for ids, want in (([1, 2], [1, 2]), (np.array([5, (1 << 32) + 6, -1]), [5, 6, 0xFFFFFFFF]), (np.array([7, -2], dtype=np.int32), [7, 0xFFFFFFFE]),
+                      (np.array([3.0]), [3]), ((), [])):
+        assert g.decode(ids) == b"text" and got[-1].dtype == np.uint32 and got[-1].tolist() == want
+    for bad in ([-1], [1 << 32]):
+        with pytest.raises(OverflowError):
+            g.decode(bad)
