@@ -47,7 +47,7 @@ class Tokenizer:
 
     def _ensure(self, n_bytes):
         cap = self._cap
-        if n_bytes > cap:
+        if 0 < cap < n_bytes:                    # (no cap: the handle is closed, as the call that follows will say)
             while cap < n_bytes:
                 cap *= 2
             self._g.set_max_bytes(cap)

@@ -79,3 +79,21 @@ def test_ids_of_other_types_in_gtok_decode():
     for bad in ([-1], [1 << 32]):
         with pytest.raises(OverflowError):
             g.decode(bad)
+
+
+def test_staging_on_a_closed_handle():
+    """The library answers no cap for a closed handle: an error, not an endless search for a cap that is large enough."""
+    assert child("""
+import faulthandler
+faulthandler.dump_traceback_later(20, exit=True)
+from graphtok_b200 import GTok, GTokError, load_lib
+from graphtok_b200.gpu_bpe_tokenizer import Tokenizer
+t = Tokenizer.__new__(Tokenizer)
+t._g = GTok.__new__(GTok)
+t._g.lib, t._g.handle = load_lib(), None
+for call in (lambda: t.bench_stage("text"), lambda: t.bench_stage_batch(["text"])):
+    try:
+        call()
+    except GTokError:
+        print("refused", end=" ")
+""").split() == ["refused"] * 2
