@@ -3195,6 +3195,10 @@ GTOK_DEV void miss_teams(Blk& blk, const EncodeArgs& a, MissSmem& sm, const unsi
 GTOK_DEV uint32_t team_take(uint32_t max_len) {
     return (max_len > static_cast<uint32_t>(kMedSplit) ? 2u : max_len > static_cast<uint32_t>(kShortWordMax) ? 4u : 8u) * kWarps;
 }
+// The single-block kernel's one list: the length class of its calls, from the longest pre-token in it.
+GTOK_DEV uint32_t one_list_max_len(uint32_t longest) {
+    return longest > static_cast<uint32_t>(kMedSplit) ? kMedWordMax : longest > static_cast<uint32_t>(kShortWordMax) ? kMedSplit : kShortWordMax;
+}
 // Whether a text's pre-tokens of 17..64 bytes are merged by teams: while they make at most one call a block, the kernel lasts as
 // long as one call and the chain counts; beyond, instructions do.  Merge kernel, teams / one thread a pre-token (592 blocks):
 // multilingual text of 0.1 MB 34 / 58 us, 1.2 MB 44 / 65, 2.4 MB (some 550 calls) 63 / 67, 4.5 MB 97 / 69; code and CJK

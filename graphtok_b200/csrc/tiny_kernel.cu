@@ -87,8 +87,7 @@ __global__ void __launch_bounds__(kThreads, 1) tiny_kernel(const __grid_constant
             if (mx) atomicMax(&s_maxlen, mx);
         }
         __syncthreads();
-        const uint32_t longest = s_maxlen;
-        const uint32_t max_len = longest > static_cast<uint32_t>(kMedSplit) ? kMedWordMax : longest > static_cast<uint32_t>(kShortWordMax) ? kMedSplit : kShortWordMax;
+        const uint32_t max_len = one_list_max_len(s_maxlen);
         for (uint32_t first = 0; first < n_miss; first += kThreads) miss_teams(blk, a, ms, a.gmiss, 1, first, n_miss, kThreads, max_len);
         for (uint32_t li = 0; li < n_long; ++li) long_word(blk, a, ms, li);
     }

@@ -153,10 +153,12 @@ void gtok_emul_destroy(void* h) { delete static_cast<Emul*>(h); }
 
 // force_non_monotone: bit 0 treats the vocabulary as non-monotone (exercises the one-merge-per-round path),
 // bit 1 matches added-token literals by the trie walk (the path of vocabularies with too many literal lengths to hash)
+// form: how unknown pre-tokens of 2..64 bytes are merged: 0 one thread a pre-token, 1 by teams (the merge kernel takes either, by the
+// text's size), 2 by teams from the one list of all lengths that the single-block kernel has
 // Returns the token count, or -(error bits) when the kernels flagged an error.
 int64_t gtok_emul_encode(void* h, const uint8_t* text, uint32_t n, const uint32_t* doc_off, uint32_t n_docs,
                          uint32_t* out, uint32_t cap, uint32_t* out_doc_tok, uint32_t* bmask_out, int reverse,
-                         int force_non_monotone) {
+                         int force_non_monotone, int form) {
     Emul* e = static_cast<Emul*>(h);
     using namespace gtok;
     const uint32_t n_tiles = (n + kTile - 1) / kTile;
@@ -189,6 +191,7 @@ int64_t gtok_emul_encode(void* h, const uint8_t* text, uint32_t n, const uint32_
     a.glong_cnt = glong.data() + static_cast<size_t>(n_tiles + 1) * kLongPerTile * 2;
     a.out_tokens = out; a.out_cap = cap; a.status = status;
     a.tb = e->tb;
+    a.one_list = form == 2 ? 1u : 0u;
     if (force_non_monotone & 1) a.tb.monotone = 0;
     if (force_non_monotone & 2) a.tb.lit_n_lens = 0;            // added-token literals by the trie walk instead of the hashed table
     CpuBlk blk;
@@ -214,18 +217,24 @@ int64_t gtok_emul_encode(void* h, const uint8_t* text, uint32_t n, const uint32_
         std::memset(sm, 0xCD, sizeof *sm);
         for (int i = 0; i < 256; ++i) sm->b2i[i] = a.tb.byte_to_id[i];
         const uint32_t n_miss = ctl[CTL_NMISS], n_med = ctl[CTL_NMED], n_med1 = ctl[CTL_NMED1], n_med2 = ctl[CTL_NMED2], n_long = ctl[CTL_NLONG];
-        // (the runs in order merge by teams, the reversed ones a thread a pre-token, whatever the size; the kernel takes one or the other by size)
         auto merge = [&](const unsigned long long* list, int dir, uint32_t count, uint32_t batch, uint32_t max_len, uint32_t take) {
-            if (!reverse) take = team_take(max_len);
+            if (form) take = team_take(max_len);
             for (uint32_t first = 0; first < count; first += take) {
-                if (reverse) miss_batch(blk, a, *sm, list, dir, first, count, batch, max_len, take);
-                else miss_teams(blk, a, *sm, list, dir, first, count, take, max_len);
+                if (form) miss_teams(blk, a, *sm, list, dir, first, count, take, max_len);
+                else miss_batch(blk, a, *sm, list, dir, first, count, batch, max_len, take);
             }
         };
-        merge(a.gmed, 1, n_med, kMedBatchA, kMedWordMax, kMedBatchA);
-        merge(a.gmed1, 1, n_med1, kMedBatchA1, kMedSplit1, kMedBatchA1);
-        merge(a.gmed + (a.gmed_cap - 1), -1, n_med2, kMedBatchB, kMedSplit, a.tb.ignore_merges ? kMedTakeB : kMedBatchB);
-        merge(a.gmiss, 1, n_miss, kMissBatch, kShortWordMax, kMissBatch);
+        if (form == 2) {
+            uint32_t longest = 0;
+            for (uint32_t i = 0; i < n_miss; ++i) longest = std::max(longest, static_cast<uint32_t>(a.gmiss[i] >> 32));
+            const uint32_t max_len = one_list_max_len(longest);
+            for (uint32_t first = 0; first < n_miss; first += kThreads) miss_teams(blk, a, *sm, a.gmiss, 1, first, n_miss, kThreads, max_len);
+        } else {
+            merge(a.gmed, 1, n_med, kMedBatchA, kMedWordMax, kMedBatchA);
+            merge(a.gmed1, 1, n_med1, kMedBatchA1, kMedSplit1, kMedBatchA1);
+            merge(a.gmed + (a.gmed_cap - 1), -1, n_med2, kMedBatchB, kMedSplit, a.tb.ignore_merges ? kMedTakeB : kMedBatchB);
+            merge(a.gmiss, 1, n_miss, kMissBatch, kShortWordMax, kMissBatch);
+        }
         for (uint32_t li = 0; li < n_long; ++li) long_word(blk, a, *sm, li);
         delete sm;
     }

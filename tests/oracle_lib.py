@@ -166,35 +166,47 @@ class Emul:
         self.lib.gtok_emul_create.argtypes = [ctypes.c_char_p, ctypes.c_char_p, ctypes.c_uint32]
         self.lib.gtok_emul_encode.restype = ctypes.c_int64
         self.lib.gtok_emul_encode.argtypes = [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_uint32, ctypes.c_void_p, ctypes.c_uint32,
-                                              ctypes.c_void_p, ctypes.c_uint32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int]
+                                              ctypes.c_void_p, ctypes.c_uint32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int]
         err = ctypes.create_string_buffer(512)
         self.h = self.lib.gtok_emul_create(os.fsencode(tokenizer_json), err, 512)
         if not self.h:
             raise RuntimeError("emul: " + err.value.decode())
 
-    def encode(self, data, offsets=None, reverse=False, non_monotone=False, want_starts=False, trie=False):
+    #: ways to merge unknown pre-tokens -> emul.cc's number
+    FORMS = {"threads": 0, "teams": 1, "one list": 2}
+    ONE_LIST_MOST = 2048         # bytes: what the single-block kernel, the one with one list, takes
+
+    def encode(self, data, offsets=None, reverse=False, non_monotone=False, want_starts=False, trie=False, form=None):
+        """`form`: one of FORMS; None: all that the text's size has, which have to agree."""
         data = bytes(data)
+        forms = [form] if form else [f for f in self.FORMS if f != "one list" or (offsets is None and len(data) <= self.ONE_LIST_MOST)]
+        results = [self._encode(data, offsets, reverse, non_monotone, want_starts, trie, self.FORMS[f]) for f in forms]
+        for f, r in zip(forms[1:], results[1:]):
+            if not all(np.array_equal(x, y) for x, y in zip(r, results[0])):
+                raise AssertionError("merging by %s gives other ids than by %s" % (f, forms[0]))
+        return results[0][0] if len(results[0]) == 1 else tuple(results[0])
+
+    def _encode(self, data, offsets, reverse, non_monotone, want_starts, trie, form):
         out = np.empty(len(data) + 16, dtype=np.uint32)
         bm = np.zeros((len(data) + 4095) // 4096 * 128 + 8, dtype=np.uint32)
+        flags = (int(reverse), int(non_monotone) | (2 if trie else 0), form)
         doc = None
         if offsets is not None:
             offsets = np.ascontiguousarray(offsets, dtype=np.uint32)
             doc = np.zeros(offsets.size, dtype=np.uint32)
             n = self.lib.gtok_emul_encode(self.h, data, len(data), offsets.ctypes.data, offsets.size - 1, out.ctypes.data, out.size,
-                                          doc.ctypes.data, bm.ctypes.data, int(reverse), int(non_monotone) | (2 if trie else 0))
+                                          doc.ctypes.data, bm.ctypes.data, *flags)
         else:
-            n = self.lib.gtok_emul_encode(self.h, data, len(data), None, 1, out.ctypes.data, out.size, None, bm.ctypes.data,
-                                          int(reverse), int(non_monotone) | (2 if trie else 0))
+            n = self.lib.gtok_emul_encode(self.h, data, len(data), None, 1, out.ctypes.data, out.size, None, bm.ctypes.data, *flags)
         if n < 0:
             raise RuntimeError("emulated kernels flagged error bits %d" % -n)
-        ids = out[:n].copy()
-        res = [ids]
+        res = [out[:n].copy()]
         if offsets is not None:
             res.append(doc)
         if want_starts:
             bits = np.unpackbits(bm.view(np.uint8), bitorder="little")[:len(data)]
             res.append(np.nonzero(bits)[0].astype(np.uint32))
-        return res[0] if len(res) == 1 else tuple(res)
+        return res
 
     def decode(self, ids, cap=None, reverse=False):
         """decode_tile over the ids; returns (bytes or None when `cap` is too small, byte count, error bits)."""
