@@ -66,17 +66,21 @@ def test_utf8_form(utf8, width, kind, n):
             assert utf8.size(units.ctypes.data, n, kind) == 0xFFFFFFFFFFFFFFFF
 
 
-@pytest.fixture(scope="module", params=["extension", "ctypes"])
-def tok(request):
-    """A tokenizer that goes by the extension, and one that goes by ctypes as where the extension was not built."""
+def _tokenizer(family, route):
+    """A tokenizer that goes by the extension, or one that goes by ctypes as where the extension was not built."""
     from graphtok_b200.ctypes_host import CtypesHost
     from graphtok_b200.gpu_bpe_tokenizer import Tokenizer
-    t = Tokenizer(tiny_vocab("llama3"))
-    if request.param == "ctypes":
+    t = Tokenizer(tiny_vocab(family))
+    if route == "ctypes":
         t._host = t._g.host = CtypesHost(t._g.lib)
     elif isinstance(t._host, CtypesHost):
         pytest.skip("the extension is not built here")
     return t
+
+
+@pytest.fixture(scope="module", params=["extension", "ctypes"])
+def tok(request):
+    return _tokenizer("llama3", request.param)
 
 
 # sizes: single-block route and its limit, one copy step and several, the size from which characters are shared among
@@ -107,6 +111,53 @@ def test_batch_of_mixed_objects(tok, oracles, docs, longest):
     assert np.array_equal(ids, np.concatenate(want))
     dev, dev_off = tok.encode_batch_to_device(texts)
     assert np.array_equal(dev.cpu().numpy(), ids.astype(np.int32)) and dev_off.cpu().tolist() == off.tolist()
+
+
+NFC_TEXTS = {
+    "nothing to do": "plain words " * 40,
+    "composed": "Cafe\u0301 a\u0323\u0302 " * 60,
+    "growing": "\u0958\u0959 \U0001d15e" * 300,                      # more bytes than before, and more ids than there were bytes
+    "a stretch too long for the device": "q" + "\u0301\u0323" * 150 + " \u0958" * 50,
+    "empty": "",
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("route", ("extension", "ctypes"))
+def test_texts_that_normalisation_changes(oracles, route):
+    """The vocabulary that declares NFC: each text alone, as part of a batch, to the host and to the device."""
+    tok, o = _tokenizer("qwen25", route), oracles["qwen25"]
+    want = {k: o.encode(t.encode()) for k, t in NFC_TEXTS.items()}
+    assert want["growing"].size > len(NFC_TEXTS["growing"].encode())
+    for repeat in (1, 40):
+        for name, text in NFC_TEXTS.items():
+            text = text * repeat
+            expect = o.encode(text.encode()) if repeat > 1 else want[name]
+            assert np.array_equal(tok.encode_numpy(text), expect), name
+            assert np.array_equal(tok.encode_numpy(text.encode()), expect), name
+            assert np.array_equal(tok.encode_to_device(text).cpu().numpy(), expect), name
+    names = list(NFC_TEXTS) * 30
+    for chosen in (names, ["growing"] * 3, ["empty", "growing"], ["nothing to do"] * 5):
+        texts = [NFC_TEXTS[n] if i % 2 else NFC_TEXTS[n].encode() for i, n in enumerate(chosen)]
+        ids, off = tok.encode_batch(texts)
+        assert np.array_equal(ids, np.concatenate([want[n] for n in chosen])), chosen[:3]
+        assert off.tolist() == [0] + np.cumsum([want[n].size for n in chosen]).tolist()
+        dev, dev_off = tok.encode_batch_to_device(texts)
+        assert np.array_equal(dev.cpu().numpy(), ids.astype(np.int32)) and dev_off.cpu().tolist() == off.tolist()
+
+
+@pytest.mark.gpu
+def test_normalised_text_beyond_the_byte_cap(oracles):
+    """A text within the handle's cap whose normalised form is not: refused, and encoded once the cap is raised."""
+    from graphtok_b200 import GTok, GTokError
+    text = (NFC_TEXTS["growing"] * 2).encode()
+    for raise_to in (3 * len(text), 8 * len(text)):
+        g = GTok(tiny_vocab("qwen25"), max_bytes=len(text))
+        with pytest.raises(GTokError, match="-3"):
+            g.encode(text)
+        g.set_max_bytes(raise_to)
+        assert np.array_equal(g.encode(text), oracles["qwen25"].encode(text))
+        g.close()
 
 
 @pytest.mark.gpu
