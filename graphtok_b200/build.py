@@ -21,7 +21,7 @@ DATAGEN = os.path.join(HERE, "datagen", "datagen")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "-lineinfo",
-    "-Xcompiler", "-fPIC", "--shared",
+    "-Xcompiler", "-fPIC", "--shared", "--threads", "8",
     "-Xlinker", "--version-script=" + os.path.join(CSRC, "gtok.map"),
 ]
 SOURCES = ["encode_kernels.cu", "tiny_kernel.cu", "engine.cu", "gtok_abi.cc", "vocab_host.cc", "tables_build.cc", "nfc_host.cc", "host_text.cc"]
@@ -57,8 +57,9 @@ def build_lib(force=False, verbose=False):
     if not force and not _newer(LIB, deps):
         return LIB
     os.makedirs(LIB_DIR, exist_ok=True)
-    cmd = [_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB] + [os.path.join(CSRC, s) for s in SOURCES]
+    cmd = [_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB + ".part"] + [os.path.join(CSRC, s) for s in SOURCES]
     subprocess.run(cmd, check=True)
+    os.replace(LIB + ".part", LIB)               # a build that was cut short leaves no library behind
     return LIB
 
 

@@ -32,6 +32,7 @@
 // greedy lowest-rank-first rule of src/tokenizer.cu:360-580 / src/host_encode.cc:617-648;
 // the batched rounds for long pre-tokens follow the idea of src/tokenizer.cu:754-791.
 #pragma once
+#include <stddef.h>
 #include <stdint.h>
 
 #include <type_traits>

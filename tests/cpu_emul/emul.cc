@@ -5,6 +5,7 @@
 // shows up as a difference between the two), and the tiles in order.  This lets
 // the CPU test suite check the kernels' logic against the oracle without a GPU.
 // It is not part of the shipped library and not a fallback: libgtok has no CPU path.
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <memory>

@@ -1,6 +1,7 @@
 """Memory of large results: what is kept of dropped ones (CPU), and that an array's ids are its own whatever becomes of it (GPU)."""
 import ctypes
 import os
+import signal
 import subprocess
 
 import numpy as np
@@ -89,6 +90,7 @@ def test_an_upload_of_a_dropped_result(tok, oracles):
 
 
 @pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore:This process .* is multi-threaded")
 def test_a_result_in_a_forked_child(tok, oracles):
     """A child that holds a result which its parent has dropped since: still the child's own."""
     want = oracles["llama3"].encode(large(8))
@@ -96,6 +98,7 @@ def test_a_result_in_a_forked_child(tok, oracles):
     read, write = os.pipe()
     child = os.fork()
     if child == 0:
+        signal.alarm(20)
         os.read(read, 1)
         os._exit(0 if np.array_equal(ids, want) else 1)
     del ids
