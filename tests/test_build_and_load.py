@@ -4,6 +4,8 @@ import os
 import subprocess
 import sys
 
+import pytest
+
 from conftest import ROOT
 
 
@@ -57,3 +59,15 @@ def test_one_copy_of_the_library_whatever_the_library_path(built, tmp_path):
                 "paths = {line.split()[-1] for line in open('/proc/self/maps') if 'libgtok.so' in line}\n"
                 "print(kind, *paths)\n", LD_LIBRARY_PATH="%s:%s" % (tmp_path, os.environ.get("LD_LIBRARY_PATH", "")))
     assert out.split() == [type(load_lib().host).__name__, build.LIB]
+
+
+def test_no_figure_for_the_reference_without_its_encoder():
+    """The reference arm of the benchmark times the reference's own encoder or nothing."""
+    import json
+
+    import oracle_lib
+    if os.path.exists(oracle_lib.REF_SO):
+        pytest.skip("the reference's encoder is built here")
+    r = subprocess.run([sys.executable, "bench.py", "--impl", "reference", "--steps", "1", "--warmup", "1"], cwd=ROOT, stdout=subprocess.PIPE, text=True)
+    line = json.loads(r.stdout)
+    assert r.returncode == 0 and line["impl"] == "reference" and line["unavailable"] and "value" not in line
