@@ -287,6 +287,15 @@ bool narrow(const T* s, uint32_t n, uint32_t* d) {
     return (high >> 32) == 0;
 }
 
+// (the first decoding call of a handle, and one that is larger than those before, make its buffers)
+uint32_t* decode_room(void* h, uint32_t n) {
+    uint32_t* room;
+    Py_BEGIN_ALLOW_THREADS
+    room = lib.decode_room(h, n);
+    Py_END_ALLOW_THREADS
+    return room;
+}
+
 // decode(handle, ids) -> bytes; None for an `ids` that this function does not take (the caller makes a uint32 array of it)
 PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "decode(handle, ids)"); return nullptr; }
@@ -301,10 +310,12 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         n = static_cast<uint32_t>(len);
         for (Py_ssize_t i = 0; i < len; ++i)
             if (!PyLong_CheckExact(PyList_GET_ITEM(o, i))) Py_RETURN_NONE;
-        uint32_t* room = lib.decode_room(h, n);
+        uint32_t* room = decode_room(h, n);
         if (!room) return PyLong_FromLong(-1);
+        if (PyList_GET_SIZE(o) != len) Py_RETURN_NONE;              // (another thread has changed it meanwhile)
         for (Py_ssize_t i = 0; i < len; ++i) {
             int over = 0;
+            if (!PyLong_CheckExact(PyList_GET_ITEM(o, i))) Py_RETURN_NONE;
             const long long v = PyLong_AsLongLongAndOverflow(PyList_GET_ITEM(o, i), &over);
             if (over || v < 0 || v > 0xFFFFFFFFll) { fits = false; break; }
             room[i] = static_cast<uint32_t>(v);
@@ -321,7 +332,7 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         n = static_cast<uint32_t>(len);
         if (d->kind == 'u' && width == 4) ids = static_cast<const uint32_t*>(PyArray_DATA(a));
         else {
-            uint32_t* room = lib.decode_room(h, n);
+            uint32_t* room = decode_room(h, n);
             if (!room) return PyLong_FromLong(-1);
             const void* s = PyArray_DATA(a);
             Py_BEGIN_ALLOW_THREADS

@@ -97,3 +97,17 @@ for call in (lambda: t.bench_stage("text"), lambda: t.bench_stage_batch(["text"]
     except GTokError:
         print("refused", end=" ")
 """).split() == ["refused"] * 2
+
+
+def test_a_list_that_changes_while_decoding_makes_its_buffers(built):
+    """The buffers are made with the interpreter lock let go: a list that is another one afterwards goes the caller's other way."""
+    assert extension("""
+room = (ctypes.c_uint32 * 100000)()
+def decode_room(handle, n):
+    change()
+    return ctypes.addressof(room)
+stand_in(decode_room=decode_room)
+for change in (lambda: ids.clear(), lambda: ids.append(1), lambda: ids.__setitem__(99999, "x")):
+    ids = [1 << 20] * 100000
+    print(host.decode(1, ids), end=" ")
+""") == "None None None"
