@@ -625,9 +625,8 @@ struct Engine::Impl {
         }
     }
 
-    // Normalisation, in two launches: look for codepoints that can make the raw text non-NFC; if
-    // there are none (the usual case) copy text and header over as they are; else normalise.  The
-    // second and third each return at once in the case that is not theirs.
+    // Normalisation, in two launches: one looks for codepoints that can make the raw text non-NFC and moves text and header
+    // over as it goes; the other returns at once where there were none (the usual case), else it normalises and writes both again.
     void launch_normalise(Ctx* c) {
         EncodeArgs chk = c->args;
         chk.raw_docmask = nullptr;

@@ -2,9 +2,9 @@
 // what follows it in gtok.h).
 //
 // The library takes text where Python keeps it (a str's own characters, a bytes object's bytes, those of a list
-// one by one) and writes ids and bytes to the object that is returned, so a call makes no intermediate
-// Python object and no copy that the transfer to or from the GPU does not need.  Every function takes the
-// handle as an integer and answers an error of the library with its (negative) code as an int.
+// one by one) and writes ids and bytes to the object that is returned, by way of its page-locked buffers: a call
+// makes no intermediate Python object and one copy each way (a bytearray or a view is copied first).  Every
+// function takes the handle as an integer and answers an error of the library with its (negative) code as an int.
 // The module is not linked against the library: bind() takes the calls' addresses from whoever has loaded it, so
 // that there is one copy of it in the process whatever else goes by the name libgtok.so on the library path.
 #define PY_SSIZE_T_CLEAN
