@@ -80,8 +80,8 @@ def load_lib():
     lib.gtok_x_phase_clocks.argtypes = [vp, vp, i32]
     lib.gtok_x_encode_batch_to_device.restype = i32
     lib.gtok_x_encode_batch_to_device.argtypes = [vp, vp, vp, u32, vp, u32, vp]
-    lib.gtok_x_order_after.restype = i32
-    lib.gtok_x_order_after.argtypes = [vp, vp]
+    lib.gtok_x_result_stream.restype = i32
+    lib.gtok_x_result_stream.argtypes = [vp, vp]
     lib.gtok_x_set_max_bytes.restype = u32
     lib.gtok_x_set_max_bytes.argtypes = [vp, u32]
     lib.gtok_x_work_stats.restype = i32

@@ -31,8 +31,8 @@ public:
     int64_t encode_batch(const uint8_t* bytes, const uint32_t* doc_off, uint32_t n_docs, uint32_t cap_bytes,
                          uint32_t* out_tokens, uint32_t out_cap, uint32_t* out_doc_tok, bool out_on_device = false);
 
-    // The next result that goes to device memory is written after the work queued on `stream` (of the current device) so far.
-    int order_after(void* stream);
+    // What the next encoding call writes to device memory is written behind the work queued on `stream` (of the current device).
+    int result_stream(void* stream);
 
     // The same call in steps, for callers that hold text in pieces (a list of strings) or make the result's memory
     // themselves once its size is known:

@@ -343,11 +343,11 @@ int64_t gtok_x_decode(void* handle, const uint32_t* ids, uint32_t n, uint8_t* ou
     } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }
 }
 
-int32_t gtok_x_order_after(void* handle, void* cuda_stream) {
+int32_t gtok_x_result_stream(void* handle, void* cuda_stream) {
     if (!handle) return -1;
     Handle* h = static_cast<Handle*>(handle);
     try {
-        const int r = h->engine->order_after(cuda_stream);
+        const int r = h->engine->result_stream(cuda_stream);
         if (r < 0) g_last_error = h->engine->last_error();
         return r;
     } catch (const std::exception& e) { g_last_error = e.what(); return -1; } catch (...) { return -1; }

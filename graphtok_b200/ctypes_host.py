@@ -76,7 +76,7 @@ class CtypesHost:
                 break
         return n if n < 0 else (out[:n].copy(), doc)
 
-    def encode_to_device(self, handle, text, grow, make):
+    def encode_to_device(self, handle, text, grow, make, queue):
         batch = text.__class__ is tuple
         if batch:
             blob, offsets = concatenated(text)
@@ -91,6 +91,8 @@ class CtypesHost:
         doc = make(offsets.size) if batch else None
         for room in (len(blob) + 16, 3 * len(blob) + 64):
             out = make(room)
+            if self.lib.gtok_x_result_stream(handle, queue()) < 0:
+                return -1
             at, most = ctypes.c_void_p(out.data_ptr()), min(room, 0xFFFFFFFF)
             if batch:
                 n = self.lib.gtok_x_encode_batch_to_device(handle, blob, offsets.ctypes.data, offsets.size - 1, at, most, ctypes.c_void_p(doc.data_ptr()))

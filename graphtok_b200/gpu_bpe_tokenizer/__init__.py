@@ -25,6 +25,17 @@ _POLICIES = {"adaptive": 0, "gpu": 1, "cpu": 2}
 _BACKENDS = ("", "auto", "off", "host", "gigatoken")
 
 
+def _device_words(n):
+    import torch
+    return torch.empty(n, dtype=torch.int32, device="cuda")
+
+
+def _queue():
+    # torch's allocator works in stream order: what used a new tensor's memory last may still be queued on this stream
+    import torch
+    return torch.cuda.current_stream().cuda_stream
+
+
 class Tokenizer:
     """One vocabulary, one GPU.  Not thread-safe (same contract as the reference, :1117-1120)."""
 
@@ -73,19 +84,11 @@ class Tokenizer:
             self._g._fail("gtok_encode_batch", out)
         return out
 
-    def _device_words(self, n):
-        import torch
-        words = torch.empty(n, dtype=torch.int32, device="cuda")
-        # torch's allocator works in stream order: what used this block last may still be queued on the current stream
-        if self._g.lib.gtok_x_order_after(self._g.handle, torch.cuda.current_stream().cuda_stream) < 0:
-            self._g._fail("gtok_x_order_after", -1)
-        return words
-
     def encode_to_device(self, text):
         """int32 torch tensor on the GPU (torch is imported only here, as in the reference :100-117)."""
         if text.__class__ is tuple:
             raise TypeError("text must be str or bytes")
-        out = self._host.encode_to_device(self._g.handle, text, True, self._device_words)
+        out = self._host.encode_to_device(self._g.handle, text, True, _device_words, _queue)
         if out.__class__ is int:
             raise RuntimeError("gtok_encode_to_device returned %d" % out)
         return out[0][:out[1]]
@@ -96,7 +99,7 @@ class Tokenizer:
         if not texts:
             import torch
             return torch.zeros(0, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
-        out = self._host.encode_to_device(self._g.handle, texts, True, self._device_words)
+        out = self._host.encode_to_device(self._g.handle, texts, True, _device_words, _queue)
         if out.__class__ is int:
             raise RuntimeError("gtok_encode_batch_to_device returned %d" % out)
         return out[0][:out[1]], out[2]

@@ -31,6 +31,7 @@ constexpr uint64_t kLargeBytes = 256 << 10;
 // The library's calls by address.
 struct Lib {
     decltype(&gtok_x_set_max_bytes) set_max_bytes;
+    decltype(&gtok_x_result_stream) result_stream;
     decltype(&gtok_x_measure) measure;
     decltype(&gtok_x_encode_measured) encode_measured;
     decltype(&gtok_x_take_ids) take_ids;
@@ -41,7 +42,7 @@ struct Lib {
 bool bound = false;
 struct Need { const char* name; void* at; };
 #define GTOK_NEED(f) {"gtok_x_" #f, &lib.f}
-const Need kNeeds[] = {GTOK_NEED(set_max_bytes), GTOK_NEED(measure), GTOK_NEED(encode_measured), GTOK_NEED(take_ids), GTOK_NEED(decode_room),
+const Need kNeeds[] = {GTOK_NEED(set_max_bytes), GTOK_NEED(result_stream), GTOK_NEED(measure), GTOK_NEED(encode_measured), GTOK_NEED(take_ids), GTOK_NEED(decode_room),
                        GTOK_NEED(decode_run), GTOK_NEED(take_bytes)};
 
 // bind(address): address(name) -> where that call of gtok.h is in the loaded library.
@@ -229,10 +230,11 @@ PyObject* py_encode_batch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return Py_BuildValue("(NN)", ids, off);
 }
 
-// encode_to_device(handle, text or tuple of texts, grow, make) -> (what make(words) returned for the ids, id count,
-// the same for the offsets or None).  make(words) returns a tensor of that many 32-bit words on the device.
+// encode_to_device(handle, text or tuple of texts, grow, make, queue) -> (what make(words) returned for the ids, id count,
+// the same for the offsets or None).  make(words) returns a tensor of that many 32-bit words on the device, queue() the
+// stream whose queued work may still use their memory.
 PyObject* py_encode_to_device(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    if (nargs != 4) { PyErr_SetString(PyExc_TypeError, "encode_to_device(handle, text or tuple, grow, make)"); return nullptr; }
+    if (nargs != 5) { PyErr_SetString(PyExc_TypeError, "encode_to_device(handle, text or tuple, grow, make, queue)"); return nullptr; }
     const bool batch = PyTuple_CheckExact(args[1]);
     Texts t;
     if (batch ? !t.place_all(args[1]) : !t.place(args[1], &t.one)) return nullptr;
@@ -264,9 +266,13 @@ PyObject* py_encode_to_device(PyObject*, PyObject* const* args, Py_ssize_t nargs
         const uint64_t room = attempt ? 3 * static_cast<uint64_t>(bytes) + 64 : static_cast<uint64_t>(bytes) + 16;
         PyObject* ids = make(room, &ids_at);
         if (!ids) { Py_XDECREF(off); return nullptr; }
+        PyObject* q = PyObject_CallNoArgs(args[4]);
+        void* stream = q ? PyLong_AsVoidPtr(q) : nullptr;
+        Py_XDECREF(q);
+        if (PyErr_Occurred()) { Py_DECREF(ids); Py_XDECREF(off); return nullptr; }
         int64_t got;
         Py_BEGIN_ALLOW_THREADS
-        got = lib.encode_measured(h, bytes, ids_at, room, off_at);
+        got = lib.result_stream(h, stream) < 0 ? -1 : lib.encode_measured(h, bytes, ids_at, room, off_at);
         Py_END_ALLOW_THREADS
         if (got == -2 && attempt == 0) { Py_DECREF(ids); continue; }
         if (got < 0) { Py_DECREF(ids); Py_XDECREF(off); return PyLong_FromLongLong(got); }
@@ -374,7 +380,7 @@ PyMethodDef kMethods[] = {
     {"encode_batch", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode_batch)), METH_FASTCALL,
      "encode_batch(handle, texts, grow) -> (uint32 ids, uint32 offsets), or an error code"},
     {"encode_to_device", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode_to_device)), METH_FASTCALL,
-     "encode_to_device(handle, text or tuple, grow, make) -> (tensor, id count, offsets or None), or an error code"},
+     "encode_to_device(handle, text or tuple, grow, make, queue) -> (tensor, id count, offsets or None), or an error code"},
     {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_decode)), METH_FASTCALL, "decode(handle, ids) -> bytes, None, or an error code"},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -32,7 +32,7 @@ void* gtok_create(const char* vocab_json_path, uint32_t max_bytes);
 int32_t gtok_encode(void* handle, const uint8_t* text, uint32_t len, uint32_t* out, uint32_t max_out);
 
 /* src/gtok_shim.cc:209-236.  As gtok_encode, ids copied device-to-device into out_dev, which they are in
- * when the call returns.  No queued work may still use out_dev (or see gtok_x_order_after). */
+ * when the call returns.  No queued work may still use out_dev (or see gtok_x_result_stream). */
 int32_t gtok_encode_to_device(void* handle, const uint8_t* text, uint32_t len, void* out_dev, uint32_t max_out);
 
 /* src/gtok_shim.cc:246-318.  n_docs documents concatenated in concat_bytes with
@@ -99,13 +99,13 @@ int32_t gtok_x_timeline(void* handle, uint64_t* out, uint32_t max_words);
  * Tokenizer.encode_batch_to_device returns (src/python_bindings.cc:410-507); its C ABI has no such entry. */
 int32_t gtok_x_encode_batch_to_device(void* handle, const uint8_t* concat_bytes, const uint32_t* doc_byte_offsets, uint32_t n_docs,
                                       void* out_tokens_dev, uint32_t out_cap, void* out_doc_offsets_dev);
-/* The next result that this handle writes to device memory (gtok_encode_to_device,
- * gtok_x_encode_batch_to_device, gtok_x_encode_measured) is written after the work that is queued on
- * `cuda_stream` now (a cudaStream_t of the current device, NULL = its default stream): a handle works on a
- * stream of its own, so a buffer that queued work still reads or writes, such as one that an allocator
- * working in stream order has just handed out again, has to be announced so.  The call that follows waits
- * on the GPU, before its copies only.  Nothing is waited for while the stream is being captured.  0 or -1. */
-int32_t gtok_x_order_after(void* handle, void* cuda_stream);
+/* What the next encoding call on this handle writes to device memory (gtok_encode_to_device,
+ * gtok_x_encode_batch_to_device, gtok_x_encode_measured) is written behind the work that is queued on
+ * `cuda_stream` (a cudaStream_t of the current device, NULL = its default stream; it must live until that
+ * call returns): a handle works on a stream of its own, so a buffer that queued work still reads or writes,
+ * such as one that an allocator working in stream order has just handed out again, has to be announced so.
+ * The encoding does not wait, only the copies do.  Ignored while the stream is being captured.  0 or -1. */
+int32_t gtok_x_result_stream(void* handle, void* cuda_stream);
 /* Raises the handle's byte cap (the limit behind return code -3) without re-creating the handle:
  * vocabulary and tables stay, the GPU context grows at the next call that needs it.  The reference
  * has callers re-create a bigger handle (src/gtok_shim.cc:160-202), which reloads the vocabulary.

@@ -34,7 +34,7 @@ def test_no_memory_for_a_calls_notes(built):
 texts = ("a",) * 20_000_000
 used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
 resource.setrlimit(resource.RLIMIT_AS, (used + (100 << 20),) * 2)
-for call in (lambda: host.encode_batch(0, texts, False), lambda: host.encode_to_device(0, texts, False, None)):
+for call in (lambda: host.encode_batch(0, texts, False), lambda: host.encode_to_device(0, texts, False, None, None)):
     try:
         call()
     except MemoryError:
@@ -53,7 +53,7 @@ def measure(handle, pieces, n, batch):
     seen.append(ctypes.string_at(at, units))
     return -1
 stand_in(measure=measure)
-for form in (lambda b: host.encode(1, b, False), lambda b: host.encode_batch(1, (b,), False), lambda b: host.encode_to_device(1, b, False, None)):
+for form in (lambda b: host.encode(1, b, False), lambda b: host.encode_batch(1, (b,), False), lambda b: host.encode_to_device(1, b, False, None, None)):
     buf = bytearray(b"first and the rest")
     form(buf)
 buf, whole = bytearray(b"another"), bytearray(b"under a view")
