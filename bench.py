@@ -259,10 +259,10 @@ def decode_numbers(g, doc, flush, reps=20):
 
 def small_input_latency(path, doc, enc, reps=60):
     """p50 of gtok_encode (host buffers) on short prefixes of the workload, on a handle created for 64 KB
-    inputs and on one created for 8 MiB (what a serving process keeps), beside the reference's CPU
+    inputs and on one created for 8 MiB (what a serving process keeps), beside the CPU
     encoder on the same prefixes: what a short prompt costs, and where the two cross."""
     from graphtok_b200 import GTok
-    res = {"what": "gtok_encode with host buffers on prefixes of the workload document; cpu = the reference's host encoder on this box, one thread"}
+    res = {"what": "gtok_encode with host buffers on prefixes of the workload document; cpu = the encoder of cpu_baseline on this box, one thread"}
     prefixes = {}
     for nb in (64, 1024, 4096, 16384, 65536):
         b = bytes(doc[:nb])
